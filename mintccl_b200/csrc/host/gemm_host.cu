@@ -390,6 +390,29 @@ int mt_gemm_rs_mxfp8(MtComm* c, void* stream, const void* const* A, const void* 
   return gemm_rs_impl(c, stream, A, B, out, stage_off, flags_off, epoch, M, N, K, nred, nctas, true, sfa, sfb);
 }
 
+// x (dtype 0 fp32, 1 fp16, 2 bf16; 16-byte aligned) -> e4m3 payload and one ue8m0 scale per 32 consecutive elements.
+int mt_mxfp8_quantize(void* stream, int dtype, const void* x, void* data, void* scale, uint64_t nelems) {
+  if (nelems % 32) return fail("MXFP8 tensors hold whole blocks of 32 elements");
+  if (dtype < 0 || dtype > 2) return fail("MXFP8 quantisation takes fp32, fp16 and bf16");
+  if (((uintptr_t)x & 15) || ((uintptr_t)data & 7)) return fail("MXFP8 quantisation needs a 16-byte aligned input");
+  if (nelems == 0) return 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  cudaError_t e = mt::launch_mx_quant(dtype, x, data, scale, nelems, sm_count(dev), (cudaStream_t)stream);
+  if (e != cudaSuccess) return fail(std::string("mxfp8 quantise launch: ") + cudaGetErrorString(e));
+  return 0;
+}
+
+// Row-major scales [rows, K / 32] -> the tiled layout mt_gemm_mxfp8 reads (rows a multiple of 128, K of 128).
+int mt_mxfp8_tile_scales(void* stream, const void* in, void* out, uint64_t rows, uint64_t kb) {
+  if (rows % 128 || kb % 4 || rows / 128 > 65535 || kb / 4 > (1u << 30)) return fail("scales: rows a multiple of 128, K of 128");
+  if (((uintptr_t)in | (uintptr_t)out) & 3) return fail("scales must be 4-byte aligned");
+  if (rows == 0 || kb == 0) return 0;
+  cudaError_t e = mt::launch_mx_tile(in, out, (uint32_t)(rows / 128), (uint32_t)(kb / 4), (cudaStream_t)stream);
+  if (e != cudaSuccess) return fail(std::string("scale tiling launch: ") + cudaGetErrorString(e));
+  return 0;
+}
+
 // Sum of MXFP8 tensors (e4m3 payload + ue8m0 scale per 32 elements) over all ranks.  op 0: all-reduce into
 // (data_out_off, scale_out_off) of every rank; op 1: reduce-scatter, shard `rank` into the local outputs.
 int mt_mxfp8_reduce(MtComm* c, void* stream, int op, uint64_t data_in_off, uint64_t scale_in_off,

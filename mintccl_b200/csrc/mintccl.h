@@ -140,6 +140,10 @@ int mt_gemm_rs_mxfp8(MtComm* c, void* stream, const void* const* A, const void* 
 int mt_mxfp8_reduce(MtComm* c, void* stream, int op, uint64_t data_in_off, uint64_t scale_in_off,
                     uint64_t data_out_off, uint64_t scale_out_off, void* const* data_out, void* const* scale_out,
                     uint64_t nelems, int nctas);
+// MXFP8 encoding on the current device: payload and scales of x (dtype 0 fp32, 1 fp16, 2 bf16), and row-major scales
+// [rows, kb] -> the tiled layout of mt_gemm_mxfp8.
+int mt_mxfp8_quantize(void* stream, int dtype, const void* x, void* data, void* scale, uint64_t nelems);
+int mt_mxfp8_tile_scales(void* stream, const void* in, void* out, uint64_t rows, uint64_t kb);
 
 // ---- device-wait self test: a wait nothing satisfies must time out and report, not hang -----------
 int mt_test_wait_timeout(MtComm* c, void* stream);

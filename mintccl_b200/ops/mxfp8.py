@@ -32,8 +32,39 @@ def scale_to_float(scale: torch.Tensor) -> torch.Tensor:
     return torch.pow(2.0, scale.float() - 127.0)
 
 
+def _plain_cuda(t: torch.Tensor) -> bool:
+    """A tensor whose memory a kernel may be pointed at: not a subclass, not traced, vmapped or under a dispatch mode
+    (those go through the torch expressions below)."""
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.layout is torch.strided
+            and not torch.compiler.is_compiling() and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+            and not t.is_neg() and torch._C._len_torch_dispatch_stack() == 0)
+
+
+def _native_quantize(flat: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """One kernel (``csrc/kernels/mxfp8_quant.cu``) for contiguous ``[blocks, 32]`` on the GPU."""
+    if flat.data_ptr() % 16:
+        flat = flat.clone()      # a slice that starts off a 16-byte boundary
+    n = flat.numel()
+    data = torch.empty(n, device=flat.device, dtype=torch.uint8)
+    scale = torch.empty(n // BLOCK, device=flat.device, dtype=torch.uint8)
+    with torch.cuda.device(flat.device):
+        stream = torch.cuda.current_stream().cuda_stream
+        if N.lib().mt_mxfp8_quantize(stream, _QUANT_DT[flat.dtype], flat.data_ptr(), data.data_ptr(), scale.data_ptr(), n) < 0:
+            raise RuntimeError(f"mt_mxfp8_quantize: {N.last_error()}")
+    return data, scale
+
+
+_QUANT_DT = {torch.float32: N.DT_F32, torch.float16: N.DT_F16, torch.bfloat16: N.DT_BF16}
+
+
 def quantize_mxfp8(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """fp32/bf16/fp16 tensor (numel a multiple of 32) -> (payload uint8 [numel], scales uint8 [numel / 32])."""
+    if x.dtype in _QUANT_DT and _plain_cuda(x):
+        return _native_quantize(x.detach().reshape(-1, BLOCK).contiguous())
+    return _torch_quantize(x)
+
+
+def _torch_quantize(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     flat = x.detach().float().reshape(-1, BLOCK)
     scale = scale_for_amax(flat.abs().amax(dim=1))
     q = (flat / scale_to_float(scale)[:, None]).to(torch.float8_e4m3fn)
@@ -122,6 +153,18 @@ def tile_scales(scale: torch.Tensor) -> torch.Tensor:
     rows, kb = scale.shape
     if rows % 128 or kb % 4:
         raise ValueError("rows must be a multiple of 128 and K of 128")
+    if (scale.dtype is torch.uint8 and scale.is_contiguous() and scale.numel() and scale.data_ptr() % 4 == 0
+            and rows < 128 << 16 and _plain_cuda(scale)):
+        out = torch.empty(rows * kb, device=scale.device, dtype=torch.uint8)
+        with torch.cuda.device(scale.device):
+            if N.lib().mt_mxfp8_tile_scales(torch.cuda.current_stream().cuda_stream, scale.data_ptr(), out.data_ptr(), rows, kb) < 0:
+                raise RuntimeError(f"mt_mxfp8_tile_scales: {N.last_error()}")
+        return out
+    return _torch_tile_scales(scale)
+
+
+def _torch_tile_scales(scale: torch.Tensor) -> torch.Tensor:
+    rows, kb = scale.shape
     t = scale.view(rows // 128, 4, 32, kb // 4, 4)       # [R, r/32, r%32, KB, kb%4]
     return t.permute(0, 3, 2, 1, 4).contiguous().view(-1)  # [R, KB, r%32, r/32, kb%4]
 
