@@ -106,6 +106,16 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(const void* smem_tile) 
   const uint64_t addr = (uint64_t)(smem_u32(smem_tile) >> 4) & 0x3fffull;
   return addr | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
+// The same for an MN-major tile (the operand is stored transposed: K rows of contiguous M or N): chunks of 64 columns,
+// each `k` rows of 128 bytes with the 128-byte swizzle, one chunk after the other.  The leading byte offset is the
+// distance of the chunks, the stride byte offset that of groups of 8 K rows (1024 bytes); a step of 16 along K adds
+// 16 rows (128 units of 16 bytes) to the address.
+__device__ __forceinline__ uint64_t make_smem_desc_mn_sw128(const void* smem_tile, uint32_t chunk_bytes) {
+  const uint64_t addr = (uint64_t)(smem_u32(smem_tile) >> 4) & 0x3fffull;
+  return addr | ((uint64_t)(chunk_bytes >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+// Bits of the instruction descriptor that say "A (B) is MN-major".
+constexpr uint32_t kIdescTransA = 1u << 15, kIdescTransB = 1u << 16;
 // Instruction descriptor: fp32 accumulate, bf16 A and B, both K-major, dense, N and M of the tile.
 __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);

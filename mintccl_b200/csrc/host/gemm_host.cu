@@ -16,6 +16,18 @@ namespace {
 constexpr int kBM = 128, kBN = 256, kBK = 64;
 constexpr int kPairDefault = 1;  // plain GEMMs on CTA pairs unless MINTCCL_GEMM_PAIR says otherwise
 
+// The encoder wants a current context.  A thread whose first CUDA call this is has none yet (autograd's backward
+// threads): bind its device and try again.
+template <class F>
+CUresult with_context(F encode) {
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+  }
+  return r;
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -30,10 +42,25 @@ int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint
   cuuint64_t strides[1] = {K * esz};
   cuuint32_t box[2] = {(cuuint32_t)(fp8 ? 128 : kBK), box_rows};  // 128 bytes per row either way
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims, strides, box, estr,
+  CUresult r = with_context([&] { return enc(map, fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled failed: CUresult " + std::to_string((int)r));
+  return 0;
+}
+
+// [K, cols] bf16 row-major (an operand stored transposed), boxes of 64 columns x 64 K rows, 128-byte swizzle.
+int make_map_t(CUtensorMap* map, const void* base, uint64_t K, uint64_t cols) {
+  static EncodeTiledFn enc = (EncodeTiledFn)mthost::driver_entry("cuTensorMapEncodeTiled");
+  if (!enc) return fail("cuTensorMapEncodeTiled not available");
+  if (((uintptr_t)base & 15) || (cols * 2) % 16) return fail("GEMM operands must be 16-byte aligned with rows a multiple of 16 bytes");
+  cuuint64_t dims[2] = {cols, K};
+  cuuint64_t strides[1] = {cols * 2};
+  cuuint32_t box[2] = {64, (cuuint32_t)kBK};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = with_context([&] { return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
+  if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled (transposed) failed: CUresult " + std::to_string((int)r));
   return 0;
 }
 
@@ -46,8 +73,8 @@ int make_sf_map(CUtensorMap* map, const void* base, uint64_t atoms) {
   cuuint64_t strides[1] = {512};
   cuuint32_t box[2] = {128, 1};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = with_context([&] { return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled (scales) failed: CUresult " + std::to_string((int)r));
   return 0;
 }
@@ -109,20 +136,22 @@ static int pick_bn(int row_tiles, int N, int nclusters, bool fp8) {
 }
 
 static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N,
-                     int K, int ldc, int nctas, bool fp8) {
+                     int K, int ldc, int nctas, bool fp8, bool ta = false, bool tb = false) {
   int dev = 0;
   cudaGetDevice(&dev);
+  const int row_tiles = (M + 255) / 256;
   int ncl = (nctas > 0 ? nctas : sm_count(dev)) / 2;
   {
     const int fit = mt::gemm_pair_max_clusters(mt::MODE_PLAIN, fp8);
     if (fit > 0 && ncl > fit) ncl = fit;
   }
-  const int bn = pick_bn(M / 256, N, ncl, fp8);
+  const int bn = pick_bn(row_tiles, N, ncl, fp8);
   mt::GemmMaps maps;
   mt::PairSfMaps sf;
   memset(&maps, 0, sizeof(maps));
   memset(&sf, 0, sizeof(sf));
-  if (make_map(&maps.a[0], A, M, K, 128, fp8) || make_map(&maps.b[0], B, N, K, bn / 2, fp8)) return -1;
+  if (ta ? make_map_t(&maps.a[0], A, K, M) : make_map(&maps.a[0], A, M, K, 128, fp8)) return -1;
+  if (tb ? make_map_t(&maps.b[0], B, K, N) : make_map(&maps.b[0], B, N, K, bn / 2, fp8)) return -1;
   maps.a2[0] = maps.a[0];
   if (fp8) {
     if (make_sf_map(&sf.sfa[0], sfa, (uint64_t)(M / 128) * (K / 128)) ||
@@ -137,9 +166,11 @@ static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B
   a.K = K;
   a.ldc = ldc;
   a.nranks = 1;
+  a.ta = ta;
+  a.tb = tb;
   a.raster = raster_for(M, N, K, fp8 ? 1 : 2) / 2;
   a.timeout_ns = 4000000000ull;
-  const int tiles = (M / 256) * (N / bn);
+  const int tiles = row_tiles * (N / bn);
   int nclusters = (nctas > 0 ? nctas : sm_count(dev)) / 2;
   if (nclusters > tiles) nclusters = tiles;
   if (nclusters < 1) nclusters = 1;
@@ -185,6 +216,16 @@ int mt_gemm(void* stream, const void* A, const void* B, void* C, int M, int N, i
   mthost::stat_add(mthost::ST_GEMM, (uint64_t)(2.0 * M * N * K));
   return 0;
 }
+
+// C[M, N] = A * B in bf16 with fp32 accumulation, where either operand may be stored transposed: A as [K, M] (ta) or
+// [M, K], B as [K, N] (tb) or [N, K].  Always on CTA pairs.
+int mt_gemm_t(void* stream, const void* A, const void* B, void* C, int M, int N, int K, int ta, int tb) {
+  if (check_shape(M, N, K, 1)) return -1;
+  if ((uintptr_t)C & 15) return fail("C must be 16-byte aligned");
+  return gemm_pair(stream, A, nullptr, B, nullptr, C, M, N, K, N, 0, false, ta != 0, tb != 0);
+}
+// Do problems of `rows` rows per rank run on CTA pairs (the kernels that take a transposed B)?
+int mt_gemm_uses_pair(int rows) { return use_pair(rows) ? 1 : 0; }
 
 // C[M, ldc] (bf16) = (A * SFA)[M, K] * (B * SFB)[N, K]^T for MXFP8 operands: e4m3 payload, ue8m0 scales per 32
 // elements along K.  The scales are given in the tiled layout the tensor core reads: [rows / 128][K / 128][512]
@@ -335,10 +376,20 @@ int mt_ag_gemm_mxfp8(MtComm* c, void* stream, const void* const* a_shard, const 
 // before the first call.  `nred`: CTAs that only reduce (the others join them when their tiles are done).
 static int gemm_rs_impl(MtComm* c, void* stream, const void* const* A, const void* const* B, void* const* out,
                         uint64_t stage_off, uint64_t flags_off, uint64_t epoch, int M, int N, int K, int nred, int nctas,
-                        bool fp8, const void* const* sfa, const void* const* sfb) {
+                        bool fp8, const void* const* sfa, const void* const* sfb, bool tb = false) {
   mt::GemmArgs a;
   if (fp8 && K % 128) return fail("MXFP8: K must be a multiple of 128");
   if (fused_common(c, a, M, N, K, flags_off, epoch)) return -1;
+  if (c->nranks == 1) {
+    // nothing to reduce: the product itself, without the staging area and the reducers' pass over it (8192 x 4096 x 1792:
+    // 128 us with them, 83 without).  The sum of one bf16 partial tile is that tile, so the bytes are the same.
+    if ((uintptr_t)out[0] & 15) return fail("out must be 16-byte aligned");
+    const int rc = tb ? gemm_pair(stream, A[0], nullptr, B[0], nullptr, out[0], M, N, K, N, nctas, false, false, true)
+                      : (fp8 ? mt_gemm_mxfp8(stream, A[0], sfa[0], B[0], sfb[0], out[0], M, N, K, N, nctas)
+                             : mt_gemm(stream, A[0], B[0], out[0], M, N, K, N, nctas));
+    return rc;
+  }
+  if (tb && !use_pair(M / c->nranks)) return fail("a transposed B needs rows per rank that are a multiple of 256");
   int grid = nctas > 0 ? nctas : sm_count(c->device);
   if (c->emulated && grid * c->nlocal > sm_count(c->device)) grid = sm_count(c->device) / c->nlocal;
   if (nred < 0 || nred >= grid) return fail("nred out of range");
@@ -361,11 +412,12 @@ static int gemm_rs_impl(MtComm* c, void* stream, const void* const* A, const voi
     mt::PairSfMaps sf;
     memset(&sf, 0, sizeof(sf));
     for (int lr = 0; lr < c->nlocal; ++lr) {
-      if (make_map(&maps.b[lr], B[lr], N, K, 128, fp8)) return -1;
+      if (tb ? make_map_t(&maps.b[lr], B[lr], K, N) : make_map(&maps.b[lr], B[lr], N, K, 128, fp8)) return -1;
       if (fp8 && (make_sf_map(&sf.sfa[lr], sfa[lr], (uint64_t)(M / 128) * (K / 128)) ||
                   make_sf_map(&sf.sfb[lr], sfb[lr], (uint64_t)(N / 128) * (K / 128))))
         return -1;
     }
+    a.tb = tb;
     a.ncomm = (nred + 1) & ~1;
     const int nclusters = (grid - a.ncomm) / 2;
     if (nclusters < 1) return fail("nred out of range");
@@ -383,6 +435,11 @@ static int gemm_rs_impl(MtComm* c, void* stream, const void* const* A, const voi
 int mt_gemm_rs(MtComm* c, void* stream, const void* const* A, const void* const* B, void* const* out,
                uint64_t stage_off, uint64_t flags_off, uint64_t epoch, int M, int N, int K, int nred, int nctas) {
   return gemm_rs_impl(c, stream, A, B, out, stage_off, flags_off, epoch, M, N, K, nred, nctas, false, nullptr, nullptr);
+}
+// The same with B stored [K, N] (the backward product of a column-parallel layer).
+int mt_gemm_rs_t(MtComm* c, void* stream, const void* const* A, const void* const* B, void* const* out,
+                 uint64_t stage_off, uint64_t flags_off, uint64_t epoch, int M, int N, int K, int nred, int nctas) {
+  return gemm_rs_impl(c, stream, A, B, out, stage_off, flags_off, epoch, M, N, K, nred, nctas, false, nullptr, nullptr, true);
 }
 int mt_gemm_rs_mxfp8(MtComm* c, void* stream, const void* const* A, const void* const* sfa, const void* const* B,
                      const void* const* sfb, void* const* out, uint64_t stage_off, uint64_t flags_off, uint64_t epoch,

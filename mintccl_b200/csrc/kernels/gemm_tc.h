@@ -31,6 +31,8 @@ struct GemmArgs {
   int32_t comm_mode;                   // AG_GEMM: 0 copy-engine push (one peer per piece), 1 copy-engine pull, 2 push with plain stores,
                                        // 3 copy-engine fan-out push (every piece to all peers)
   int32_t comm_split;                  // AG_GEMM: comm CTAs that share one 128-row chunk
+  int32_t ta, tb;                      // CTA pairs, bf16: the operand is stored [K, M] / [K, N] (ta: plain GEMM only,
+                                       // tb: plain and GEMM_RS); its map then has boxes of 64 columns x 64 K rows
   int32_t raster;                      // plain GEMM: row blocks per group of the tile order (<= 1: row-major)
   uint64_t shard_off;                  // AG_GEMM pull: heap offset of every rank's own rows
   uint64_t gather_off;                 // AG_GEMM: heap offset of the gathered A buffer [M, K]
@@ -53,7 +55,7 @@ struct PairSfMaps {
 // 112 rows)
 cudaError_t launch_gemm_pair(int mode, const GemmMaps& maps, const PairSfMaps& sf, const GemmArgs& a, int nclusters,
                              int nlocal, cudaStream_t s, bool fp8, int bn = 256);
-int gemm_pair_max_clusters(int mode, bool fp8, int bn = 256);
+int gemm_pair_max_clusters(int mode, bool fp8, int bn = 256, int form = 0);
 int gemm_pair_error();   // 1 after a wait of the pair kernel expired (synchronises), -1 on a CUDA error
 
 }  // namespace mt

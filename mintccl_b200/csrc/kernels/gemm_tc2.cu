@@ -25,6 +25,11 @@
 // all CTAs) reduce this rank's rows.  The comm and reducer CTAs are the ones of gemm_tc.cu
 // (gemm_fused_parts.cuh); they come in whole clusters and never take part in a cluster barrier.
 //
+// Operands may be stored transposed (bf16; a.ta, a.tb): the backward products of a linear layer contract over the
+// dimension that is not contiguous.  TMA then fetches 64 x 64 boxes of [K, columns] and the MMA descriptors say
+// MN-major, so nothing is copied first.  Making K-major copies of the six operands of an MLP's backward pass took
+// 585 of the 1400 us of a training step (8192 x 4096 x 1792); the transposed forms run at the speed of the plain one.
+//
 // The reference has no compute kernels (README.md:5 only asks that collectives fuse with others).
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -93,19 +98,23 @@ using Tile = MtTile;
 template <int MODE, int TILE_N>
 __device__ __forceinline__ Tile tile_of(const GemmArgs& a, int lr, int t) {
   static_assert(MODE_PLAIN == MT_TILE_PLAIN && MODE_AG_GEMM == MT_TILE_AG_GEMM && MODE_GEMM_RS == MT_TILE_GEMM_RS, "mode codes");
-  return mt_fused_tile(MODE, t, a.M, a.N, a.nranks, a.rank[lr], a.raster, BM2, TILE_N);
+  // a last block of 128 rows (plain GEMM) counts as a whole one: its peer CTA loads zeros and stores nothing
+  return mt_fused_tile(MODE, t, MODE == MODE_PLAIN ? (a.M + BM2 - 1) & ~(BM2 - 1) : a.M, a.N, a.nranks, a.rank[lr], a.raster, BM2, TILE_N);
 }
 
 // TILE_N: columns of a tile, 256 or 224.  224 exists for the wave count: 8192 x 1792 (the Llama-3-8B up projection on
 // 8 ranks) is 224 tiles of 256 x 256, 3.03 waves on 74 clusters, i.e. a fourth wave for two tiles; as 256 tiles of
 // 256 x 224 it is four waves of tiles that are an eighth smaller.  bf16 only (the MXFP8 scale atoms cover 128
 // rows of B) and not for GEMM -> reduce-scatter (its staging layout is in 256-column tiles).
-template <int MODE, bool FP8, int TILE_N>
+// TA, TB: the operand is stored transposed (compile-time: choosing descriptors in the issue loops cost 7 %).
+template <int MODE, bool FP8, int TILE_N, bool TA = false, bool TB = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ PairSfMaps sfmaps, GemmArgs a) {
   static_assert(TILE_N == 256 || (TILE_N == 224 && !FP8 && MODE != MODE_GEMM_RS), "tile widths");
   constexpr int BN = TILE_N, BNC = TILE_N / 2;             // shadow the 256-column constants of the namespace
   constexpr uint32_t B_BYTES = BNC * 128;                   // a multiple of 1024: whole 128-byte swizzle atoms
+  constexpr uint32_t B_PITCH = 128 * 128;                   // a transposed B takes two whole 64-column chunks
+  constexpr uint32_t T_CHUNK = 64 * 128;                    // 64 K rows of 64 columns
   extern __shared__ uint8_t smem_raw[];
   const int lr = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -160,13 +169,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abort_flag = &ctl->abort;
 
-  const int tiles = (a.M / BM2) * (a.N / BN);
+  static_assert(!(TA || TB) || !FP8, "8-bit operands are K-major");
+  const int tiles = ((a.M + BM2 - 1) / BM2) * (a.N / BN);
   const int kblocks = a.K / BKE;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one lane, both CTAs)
     if (lane == 0) {
-      uint32_t it = 0;
+      const uint32_t empty_peer = map_to_cta(smem_u32(&ctl->empty[0]), 1), full_leader = map_to_cta(smem_u32(&ctl->full[0]), 0);
+      uint32_t s = 0, ph = 0;   // stage and its parity: running counters, no division in the issue loops
+      bool passed = false;      // the ring has been round once
       for (int t = cluster_id; t < tiles && !*abort_flag; t += nclusters) {
         const Tile tc_ = tile_of<MODE, BN>(a, lr, t);
         int arow = tc_.mb * BM2 + (int)cr * BMC;
@@ -199,21 +211,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             fence_proxy_async_global();  // peer stores (generic proxy) before our TMA reads (async proxy)
           }
         }
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
+        for (int kb = 0; kb < kblocks; ++kb) {
           if (!wait_bar(&ctl->empty[s], ph ^ 1, abort_flag, timeout_ns)) break;
           // the MMA thread's commit lands on the leader's barrier only: pass it on to the peer's producer
-          if (leader && it >= (uint32_t)STAGES) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->empty[s]), 1));
-          const uint32_t full0 = map_to_cta(smem_u32(&ctl->full[s]), 0);
-          if (leader) mbar_expect_tx(&ctl->full[s], 2 * (A_BYTES + B_BYTES + (FP8 ? SF_STAGE_BYTES : 0)));
-          tma_load_2d_pair(sA + s * A_BYTES, amap, kb * BKE, arow, full0);
-          tma_load_2d_pair(sB + s * B_BYTES, &maps.b[lr], kb * BKE, brow, full0);
+          if (leader && passed) mbar_arrive_cluster(empty_peer + s * 8);
+          const uint32_t full0 = full_leader + s * 8;
+          if (leader) mbar_expect_tx(&ctl->full[s], 2 * (A_BYTES + (TB ? B_PITCH : B_BYTES) + (FP8 ? SF_STAGE_BYTES : 0)));
+          if (TA) {
+            tma_load_2d_pair(sA + s * A_BYTES, amap, arow, kb * BKE, full0);
+            tma_load_2d_pair(sA + s * A_BYTES + T_CHUNK, amap, arow + 64, kb * BKE, full0);
+          } else {
+            tma_load_2d_pair(sA + s * A_BYTES, amap, kb * BKE, arow, full0);
+          }
+          if (TB) {
+            tma_load_2d_pair(sB + s * B_PITCH, &maps.b[lr], brow, kb * BKE, full0);
+            tma_load_2d_pair(sB + s * B_PITCH + T_CHUNK, &maps.b[lr], brow + 64, kb * BKE, full0);
+          } else {
+            tma_load_2d_pair(sB + s * B_PITCH, &maps.b[lr], kb * BKE, brow, full0);
+          }
           if (FP8) {
             // scale atoms are rows of a [atoms, 128 x u32] tensor: atom (row block of 128, K block of 128)
             uint8_t* sf = sSF + s * SF_STAGE_BYTES;
             tma_load_2d_pair(sf, &sfmaps.sfa[lr], 0, sfa_row * kblocks + kb, full0);
             tma_load_2d_pair(sf + 512, &sfmaps.sfb[lr], 0, (tc_.nb * 2) * kblocks + kb, full0);
             tma_load_2d_pair(sf + 1024, &sfmaps.sfb[lr], 0, (tc_.nb * 2 + 1) * kblocks + kb, full0);
+          }
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1;
+            passed = true;
           }
         }
       }
@@ -226,23 +252,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (one lane of the leader)
     if (leader && lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM2, BN);
-      uint32_t it = 0, tile_i = 0;
+      constexpr uint32_t idesc = make_idesc_bf16(BM2, BN) | (TA ? kIdescTransA : 0u) | (TB ? kIdescTransB : 0u);
+      constexpr uint32_t ka = TA ? 128 : 2, kb16 = TB ? 128 : 2;   // descriptor step of 16 elements along K
+      const uint64_t da0 = TA ? make_smem_desc_mn_sw128(sA, T_CHUNK) : make_smem_desc_sw128(sA);
+      const uint64_t db0 = TB ? make_smem_desc_mn_sw128(sB, T_CHUNK) : make_smem_desc_sw128(sB);
+      const uint32_t empty0 = smem_u32(&ctl->empty[0]);
+      uint32_t s = 0, ph = 0, tile_i = 0;
       for (int t = cluster_id; t < tiles && !*abort_flag; t += nclusters, ++tile_i) {
         const uint32_t as = tile_i % ACC, aph = (tile_i / ACC) & 1;
         if (!wait_bar(&ctl->acc_empty[as], aph ^ 1, abort_flag, timeout_ns)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * BN;
         bool ok = true;
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
+        for (int kb = 0; kb < kblocks; ++kb) {
           if (!wait_bar(&ctl->full[s], ph, abort_flag, timeout_ns)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint64_t da = make_smem_desc_sw128(sA + s * A_BYTES);
-          const uint64_t db = make_smem_desc_sw128(sB + s * B_BYTES);
+          // descriptor addresses are in units of 16 bytes and stay below 2^14: no carry into the other fields
+          const uint64_t da = da0 + s * (A_BYTES >> 4), db = db0 + s * (B_PITCH >> 4);
           if (FP8) {
             const uint32_t tsfa = tmem_base + 256, tsfb = tmem_base + 260;
             const uint8_t* sf = sSF + s * SF_STAGE_BYTES;
@@ -256,10 +285,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              umma_bf16_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              umma_bf16_pair(d_tmem, da + (uint64_t)(k * ka), db + (uint64_t)(k * kb16), idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
           // the stage is free (in both CTAs) once these MMAs have read it
-          umma_commit_pair(smem_u32(&ctl->empty[s]));
+          umma_commit_pair(empty0 + s * 8);
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1;
+          }
         }
         if (!ok) break;
         umma_commit_pair(smem_u32(&ctl->acc_full[as]));
@@ -298,11 +331,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         dst = (uint8_t*)a.c[lr] + (uint64_t)(tc_.mb * BM2 + (int)cr * BMC) * ld_bytes + (uint64_t)tc_.nb * BN * 2;
       }
       dst += (uint64_t)(q * 32) * ld_bytes;
+      const bool rows_out = MODE != MODE_PLAIN || tc_.mb * BM2 + (int)cr * BMC < a.M;   // M % 256 == 128: last peer has none
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN;
       const uint32_t acc_empty0 = map_to_cta(smem_u32(&ctl->acc_empty[as]), 0);
       // 4 rows per pass of 8 lanes x 16 bytes: full 128-byte lines
       // `nchunk` 16-byte pieces per row: 8 for a full block of 64 columns, 4 for the last half block of a 224 tile
       auto store_block = [&](int cb, int nchunk = 8) {
+        if (!rows_out) return;
 #pragma unroll
         for (int p = 0; p < 8; ++p) {
           const int rr = p * 4 + (lane >> 3), c16 = lane & 7;
@@ -414,31 +449,40 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
 }  // namespace pair
 
-static const void* pair_fn(int mode, bool fp8, int bn = 256) {
-  if (bn == 224) {
-    if (fp8) return nullptr;
-    if (mode == MODE_PLAIN) return (const void*)pair::gemm_pair_kernel<MODE_PLAIN, false, 224>;
-    if (mode == MODE_AG_GEMM) return (const void*)pair::gemm_pair_kernel<MODE_AG_GEMM, false, 224>;
-    return nullptr;
+// Operand forms of the bf16 kernels: 0 both K-major, 1 B stored transposed, 2 both stored transposed (plain GEMM only).
+static const void* pair_fn(int mode, bool fp8, int bn = 256, int form = 0) {
+  using pair::gemm_pair_kernel;
+  if (fp8) {
+    if (bn != 256 || form) return nullptr;
+    switch (mode) {
+      case MODE_PLAIN: return (const void*)gemm_pair_kernel<MODE_PLAIN, true, 256>;
+      case MODE_AG_GEMM: return (const void*)gemm_pair_kernel<MODE_AG_GEMM, true, 256>;
+      case MODE_GEMM_RS: return (const void*)gemm_pair_kernel<MODE_GEMM_RS, true, 256>;
+      default: return nullptr;
+    }
   }
-  switch (mode * 2 + (fp8 ? 1 : 0)) {
-    case MODE_PLAIN * 2: return (const void*)pair::gemm_pair_kernel<MODE_PLAIN, false, 256>;
-    case MODE_PLAIN * 2 + 1: return (const void*)pair::gemm_pair_kernel<MODE_PLAIN, true, 256>;
-    case MODE_AG_GEMM * 2: return (const void*)pair::gemm_pair_kernel<MODE_AG_GEMM, false, 256>;
-    case MODE_AG_GEMM * 2 + 1: return (const void*)pair::gemm_pair_kernel<MODE_AG_GEMM, true, 256>;
-    case MODE_GEMM_RS * 2: return (const void*)pair::gemm_pair_kernel<MODE_GEMM_RS, false, 256>;
-    case MODE_GEMM_RS * 2 + 1: return (const void*)pair::gemm_pair_kernel<MODE_GEMM_RS, true, 256>;
-    default: return nullptr;
+  if (mode == MODE_PLAIN) {
+    if (form == 1) return bn == 224 ? (const void*)gemm_pair_kernel<MODE_PLAIN, false, 224, false, true>
+                                    : (const void*)gemm_pair_kernel<MODE_PLAIN, false, 256, false, true>;
+    if (form == 2) return bn == 224 ? (const void*)gemm_pair_kernel<MODE_PLAIN, false, 224, true, true>
+                                    : (const void*)gemm_pair_kernel<MODE_PLAIN, false, 256, true, true>;
+    return bn == 224 ? (const void*)gemm_pair_kernel<MODE_PLAIN, false, 224> : (const void*)gemm_pair_kernel<MODE_PLAIN, false, 256>;
   }
+  if (mode == MODE_AG_GEMM && form == 0)
+    return bn == 224 ? (const void*)gemm_pair_kernel<MODE_AG_GEMM, false, 224> : (const void*)gemm_pair_kernel<MODE_AG_GEMM, false, 256>;
+  if (mode == MODE_GEMM_RS && bn == 256)
+    return form == 1 ? (const void*)gemm_pair_kernel<MODE_GEMM_RS, false, 256, false, true>
+                     : (form == 0 ? (const void*)gemm_pair_kernel<MODE_GEMM_RS, false, 256> : nullptr);
+  return nullptr;
 }
 
 // Clusters of this kernel that the device can hold at once.  The kernel is persistent (cluster i takes tiles
 // i, i + n, ...), so a grid with more clusters than fit would run its tail after the rest has finished.
-int gemm_pair_max_clusters(int mode, bool fp8, int bn) {
-  static int cached[12] = {};
-  const void* fn = pair_fn(mode, fp8, bn);
+int gemm_pair_max_clusters(int mode, bool fp8, int bn, int form) {
+  static int cached[36] = {};
+  const void* fn = pair_fn(mode, fp8, bn, form);
   if (!fn) return 0;
-  int& slot = cached[(mode * 2 + (fp8 ? 1 : 0)) * 2 + (bn == 224 ? 1 : 0)];
+  int& slot = cached[((mode * 2 + (fp8 ? 1 : 0)) * 2 + (bn == 224 ? 1 : 0)) * 3 + form];
   if (slot > 0) return slot;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::SMEM_BYTES) != cudaSuccess) return 0;
   int dev = 0, sms = 148;
@@ -472,9 +516,10 @@ int gemm_pair_max_clusters(int mode, bool fp8, int bn) {
 // Grid: 2 * nclusters GEMM CTAs followed by a.ncomm comm / reducer CTAs (even), times nlocal emulated ranks.
 cudaError_t launch_gemm_pair(int mode, const GemmMaps& maps, const PairSfMaps& sf, const GemmArgs& a, int nclusters,
                              int nlocal, cudaStream_t s, bool fp8, int bn) {
-  const void* fn = pair_fn(mode, fp8, bn);
-  if (!fn) return cudaErrorInvalidValue;
-  const int fit = gemm_pair_max_clusters(mode, fp8, bn);  // also sets the shared-memory attribute once
+  const int form = a.ta ? 2 : (a.tb ? 1 : 0);
+  const void* fn = pair_fn(mode, fp8, bn, form);
+  if (!fn || (a.ta && !a.tb)) return cudaErrorInvalidValue;
+  const int fit = gemm_pair_max_clusters(mode, fp8, bn, form);  // also sets the shared-memory attribute once
   if (fit <= 0) return cudaErrorInvalidValue;
   const int extra = mode == MODE_PLAIN ? 0 : a.ncomm;
   if (extra & 1) return cudaErrorInvalidValue;

@@ -121,6 +121,11 @@ int mt_p2p_mode(MtComm* c, void* stream, int src_rank, int dst_rank, const void*
 int mt_gemm(void* stream, const void* A, const void* B, void* C, int M, int N, int K, int ldc, int nctas);
 int mt_gemm_mxfp8(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N,
                   int K, int ldc, int nctas);
+// Operands stored transposed: A as [K, M] (ta), B as [K, N] (tb); CTA pairs only.
+int mt_gemm_t(void* stream, const void* A, const void* B, void* C, int M, int N, int K, int ta, int tb);
+int mt_gemm_uses_pair(int rows);
+int mt_gemm_rs_t(MtComm* c, void* stream, const void* const* A, const void* const* B, void* const* out,
+                 uint64_t stage_off, uint64_t flags_off, uint64_t epoch, int M, int N, int K, int nred, int nctas);
 // Plain GEMMs with M % 256 == 0 run on CTA pairs (tcgen05 cta_group::2) when MINTCCL_GEMM_PAIR is not 0; a wait
 // of that kernel that expired leaves 1 here (synchronises the device).
 int mt_gemm_pair_error(void);

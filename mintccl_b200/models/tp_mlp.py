@@ -15,7 +15,7 @@ from typing import Optional
 
 import torch
 
-from ..ops.gemm import AllGatherGemm, GemmReduceScatter, gemm
+from ..ops.gemm import AllGatherGemm, GemmReduceScatter, gemm_t
 
 
 class _MLPFunction(torch.autograd.Function):
@@ -41,14 +41,12 @@ class _MLPFunction(torch.autograd.Function):
         if n > 1:
             x = x.clone()
             x[comm.rank * (T // n):(comm.rank + 1) * (T // n)].copy_(x_shard)
-        # da = dy @ w_down            (w_down: [H, F/n])  -> B operand is w_down^T stored [F/n, H]
-        da = gemm(dy, w_down.t().contiguous())               # [T, F/n]
-        dw_down = gemm(dy.t().contiguous(), a.t().contiguous())   # [H, F/n] = dy^T @ a
+        da = gemm_t(dy, w_down, tb=True)                     # [T, F/n] = dy @ w_down       (w_down: [H, F/n])
+        dw_down = gemm_t(dy, a, ta=True, tb=True)            # [H, F/n] = dy^T @ a
         sig = torch.sigmoid(h.float())
         dh = (da.float() * (sig * (1 + h.float() * (1 - sig)))).to(torch.bfloat16)
-        dw_up = gemm(dh.t().contiguous(), x.t().contiguous())     # [F/n, H] = dh^T @ x
-        # dx = reduce_scatter(dh @ w_up)   (w_up: [F/n, H]) -> B operand [H, F/n]
-        dx_shard = mlp.gemm_rs_bwd(dh, w_up.t().contiguous())
+        dw_up = gemm_t(dh, x, ta=True, tb=True)              # [F/n, H] = dh^T @ x
+        dx_shard = mlp.gemm_rs_bwd.call_transposed(dh, w_up)      # reduce_scatter(dh @ w_up)    (w_up: [F/n, H])
         return dx_shard, dw_up, dw_down, None
 
 

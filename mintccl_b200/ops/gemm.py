@@ -45,6 +45,25 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, n
     return out
 
 
+def gemm_t(a: torch.Tensor, b: torch.Tensor, ta: bool = False, tb: bool = False) -> torch.Tensor:
+    """``op(a) @ op(b)`` with the operands as they are stored: ``a`` is ``[K, M]`` with ``ta``, else ``[M, K]``; ``b`` is
+    ``[K, N]`` with ``tb``, else ``[N, K]``.  What a backward pass needs, without transposed copies: ``tb`` for the
+    gradient of the input, both for that of the weight (``ta`` alone has no kernel)."""
+    if ta and not tb:
+        raise ValueError("gemm_t: ta goes with tb")
+    _check(a, "a")
+    _check(b, "b")
+    M, K = (a.shape[1], a.shape[0]) if ta else a.shape
+    Nn, K2 = (b.shape[1], b.shape[0]) if tb else b.shape
+    if K != K2:
+        raise ValueError("inner dimensions differ")
+    out = torch.empty(M, Nn, device=a.device, dtype=torch.bfloat16)
+    stream = torch.cuda.current_stream(a.device).cuda_stream
+    if N.lib().mt_gemm_t(stream, a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, int(ta), int(tb)) < 0:
+        raise RuntimeError(f"mt_gemm_t: {N.last_error()}")
+    return out
+
+
 class _Fused:
     def __init__(self, comm):
         self.comm = comm
@@ -204,6 +223,18 @@ class GemmReduceScatter(_Fused):
         return max(2, min(16, int(bytes_red / t / 70e9 + 0.999)))
 
     def __call__(self, a: TensorOrList, w: TensorOrList, out: Optional[TensorOrList] = None, nctas: int = 0):
+        return self._run(a, w, out, nctas, False)
+
+    def call_transposed(self, a: TensorOrList, w: TensorOrList):
+        """``reduce_scatter(a[M, K_local] @ w[K_local, N])``: ``w`` as the forward pass of a column-parallel layer holds it."""
+        rows = self.M // self.comm.world_size
+        if self.comm.world_size > 1 and not self.comm.lib.mt_gemm_uses_pair(rows):
+            # the single-CTA kernels read B along K only
+            wt = [t.t().contiguous() for t in self._lists(w)]
+            return self._run(a, wt if self.comm.emulated else wt[0], None, 0, False)
+        return self._run(a, w, None, 0, True)
+
+    def _run(self, a, w, out, nctas, tb):
         c = self.comm
         a_s, ws = self._lists(a), self._lists(w)
         rows = self.M // c.world_size
@@ -213,13 +244,14 @@ class GemmReduceScatter(_Fused):
             outs = self._lists(out)
         for t in a_s + ws + outs:
             _check(t, "operand")
-        if tuple(a_s[0].shape) != (self.M, self.K) or tuple(ws[0].shape) != (self.N, self.K):
+        if tuple(a_s[0].shape) != (self.M, self.K) or tuple(ws[0].shape) != ((self.K, self.N) if tb else (self.N, self.K)):
             raise ValueError("operand shapes do not match the plan")
         self.epoch += 1
-        rc = c.lib.mt_gemm_rs(c._handle, c._stream(), N.ptr_array([t.data_ptr() for t in a_s]),
-                              N.ptr_array([t.data_ptr() for t in ws]), N.ptr_array([t.data_ptr() for t in outs]),
-                              self._off(self.stage), self._off(self.flags), self.epoch, self.M, self.N, self.K,
-                              min(self.nred, 148 // c.nlocal - 1) if c.emulated else self.nred, nctas)
+        fn = c.lib.mt_gemm_rs_t if tb else c.lib.mt_gemm_rs
+        rc = fn(c._handle, c._stream(), N.ptr_array([t.data_ptr() for t in a_s]),
+                N.ptr_array([t.data_ptr() for t in ws]), N.ptr_array([t.data_ptr() for t in outs]),
+                self._off(self.stage), self._off(self.flags), self.epoch, self.M, self.N, self.K,
+                min(self.nred, 148 // c.nlocal - 1) if c.emulated else self.nred, nctas)
         if rc < 0:
             raise RuntimeError(f"mt_gemm_rs: {N.last_error()}")
         return outs if c.emulated else outs[0]

@@ -175,3 +175,37 @@ def test_fused_kernels_mxfp8_emulated(n):
         rows = M // n
         for r in range(n):
             torch.testing.assert_close(ys[r].float(), ref[r * rows:(r + 1) * rows], rtol=2e-2, atol=6e-2)
+
+
+@pytest.mark.parametrize("ta,tb", [(False, True), (True, True)])
+@pytest.mark.parametrize("shape", [(128, 256, 64), (384, 256, 128), (256, 1792, 192), (1920, 512, 448), (8192, 1792, 256)])
+def test_gemm_with_operands_stored_transposed(shape, ta, tb):
+    """Same product, same accumulation order as on K-major copies: the same bits on the same tiles (N = 1792 takes
+    224-column tiles where that saves a wave); M % 256 == 128 leaves the last CTA pair half empty."""
+    from mintccl_b200.ops.gemm import gemm, gemm_t
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    out = gemm_t(a.t().contiguous() if ta else a, w.t().contiguous() if tb else w, ta=ta, tb=tb)
+    torch.cuda.synchronize()
+    close(out, ref_mm(a, w), K)
+    if M % 256 == 0:
+        assert torch.equal(out, gemm(a, w))
+
+
+@pytest.mark.parametrize("n,rows", [(1, 128), (2, 256), (2, 128), (4, 256)])   # 128 rows a rank: single-CTA kernels
+def test_gemm_rs_with_a_transposed_weight(n, rows):
+    from mintccl_b200.ops.gemm import GemmReduceScatter
+    w_ = world(n)
+    M, N, K = rows * n, 512, 192
+    plan = GemmReduceScatter(w_, M, N, K)
+    for it in range(2):
+        g = torch.Generator(device="cuda").manual_seed(20 + it)
+        As = [torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16) for _ in range(n)]
+        ws = [(torch.randn(N, K, generator=g, device="cuda") * 0.05).to(torch.bfloat16) for _ in range(n)]
+        want = [t.clone() for t in plan(As, ws)]
+        got = plan.call_transposed(As, [w.t().contiguous() for w in ws])
+        w_.check()
+        for x, y in zip(got, want):
+            assert torch.equal(x, y)
