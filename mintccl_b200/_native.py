@@ -132,6 +132,8 @@ def lib():
     sig("mt_ag_gemm_mxfp8", i32, vp, vp, pp, pp, pp, pp, pp, u64, u64, u64, i32, i32, i32, i32, i32, i32)
     sig("mt_gemm_t", i32, vp, vp, vp, vp, i32, i32, i32, i32, i32)
     sig("mt_gemm_uses_pair", i32, i32)
+    sig("mt_gemm_dsilu", i32, vp, vp, vp, vp, vp, i32, i32, i32)
+    sig("mt_ag_gemm_silu", i32, vp, vp, pp, pp, pp, pp, u64, u64, u64, i32, i32, i32, i32, i32, i32, i32, u64, i32)
     sig("mt_gemm_rs_t", i32, vp, vp, pp, pp, pp, u64, u64, u64, i32, i32, i32, i32, i32)
     sig("mt_gemm_rs_mxfp8", i32, vp, vp, pp, pp, pp, pp, pp, u64, u64, u64, i32, i32, i32, i32, i32)
     sig("mt_mxfp8_reduce", i32, vp, vp, i32, u64, u64, u64, u64, pp, pp, u64, i32)

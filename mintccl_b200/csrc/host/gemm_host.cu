@@ -136,7 +136,8 @@ static int pick_bn(int row_tiles, int N, int nclusters, bool fp8) {
 }
 
 static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N,
-                     int K, int ldc, int nctas, bool fp8, bool ta = false, bool tb = false) {
+                     int K, int ldc, int nctas, bool fp8, bool ta = false, bool tb = false, int epi = mt::EPI_NONE,
+                     void* aux = nullptr) {
   int dev = 0;
   cudaGetDevice(&dev);
   const int row_tiles = (M + 255) / 256;
@@ -168,6 +169,8 @@ static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B
   a.nranks = 1;
   a.ta = ta;
   a.tb = tb;
+  a.epi = epi;
+  a.aux[0] = aux;
   a.raster = raster_for(M, N, K, fp8 ? 1 : 2) / 2;
   a.timeout_ns = 4000000000ull;
   const int tiles = row_tiles * (N / bn);
@@ -223,6 +226,12 @@ int mt_gemm_t(void* stream, const void* A, const void* B, void* C, int M, int N,
   if (check_shape(M, N, K, 1)) return -1;
   if ((uintptr_t)C & 15) return fail("C must be 16-byte aligned");
   return gemm_pair(stream, A, nullptr, B, nullptr, C, M, N, K, N, 0, false, ta != 0, tb != 0);
+}
+// C[M, N] = (A[M, K] * B[K, N]) * silu'(H[M, N]): the gradient through silu and the layer behind it.
+int mt_gemm_dsilu(void* stream, const void* A, const void* B, const void* H, void* C, int M, int N, int K) {
+  if (check_shape(M, N, K, 1)) return -1;
+  if (((uintptr_t)C | (uintptr_t)H) & 15) return fail("C and H must be 16-byte aligned");
+  return gemm_pair(stream, A, nullptr, B, nullptr, C, M, N, K, N, 0, false, false, true, mt::EPI_DSILU, (void*)H);
 }
 // Do problems of `rows` rows per rank run on CTA pairs (the kernels that take a transposed B)?
 int mt_gemm_uses_pair(int rows) { return use_pair(rows) ? 1 : 0; }
@@ -290,12 +299,22 @@ static int fused_common(MtComm* c, mt::GemmArgs& a, int M, int N, int K, uint64_
 static int ag_gemm_impl(MtComm* c, void* stream, const void* const* a_shard, const void* const* B, void* const* C,
                         uint64_t gather_off, uint64_t flags_off, uint64_t epoch, int M, int N, int K, int ldc, int ncomm,
                         int nctas, int comm_mode, uint64_t shard_off, int comm_split, bool fp8, const void* const* sfa,
-                        const void* const* sfb) {
+                        const void* const* sfb, void* const* act = nullptr) {
   mt::GemmArgs a;
   if (fp8 && K % 128) return fail("MXFP8: K must be a multiple of 128");
   if (fused_common(c, a, M, N, K, flags_off, epoch)) return -1;
   if (ldc < N || ldc % 8) return fail("ldc must be >= N and a multiple of 8");
   const int n = c->nranks;
+  if (act) {
+    for (int lr = 0; lr < c->nlocal; ++lr) {
+      if (((uintptr_t)C[lr] | (uintptr_t)act[lr]) & 15) return fail("C and the activation must be 16-byte aligned");
+      a.aux[lr] = act[lr];
+    }
+    a.epi = mt::EPI_SILU;
+    if (n == 1)   // nothing to gather (M % 256 == 128 included)
+      return gemm_pair(stream, a_shard[0], nullptr, B[0], nullptr, C[0], M, N, K, ldc, nctas, false, false, false, mt::EPI_SILU, act[0]);
+    if (!use_pair(M / n) || comm_mode == 2) return fail("the fused activation runs on CTA pairs");
+  }
   if (n == 1) ncomm = 0;
   else if (ncomm < 1 || ncomm > 64) return fail("ncomm out of range");
   int grid = nctas > 0 ? nctas : sm_count(c->device);
@@ -357,6 +376,13 @@ int mt_ag_gemm(MtComm* c, void* stream, const void* const* a_shard, const void* 
                int nctas, int comm_mode, uint64_t shard_off, int comm_split) {
   return ag_gemm_impl(c, stream, a_shard, B, C, gather_off, flags_off, epoch, M, N, K, ldc, ncomm, nctas, comm_mode,
                       shard_off, comm_split, false, nullptr, nullptr);
+}
+// The same with act[M, ldc] = silu(C) from the epilogue (C as rounded to bf16).
+int mt_ag_gemm_silu(MtComm* c, void* stream, const void* const* a_shard, const void* const* B, void* const* C, void* const* act,
+                    uint64_t gather_off, uint64_t flags_off, uint64_t epoch, int M, int N, int K, int ldc, int ncomm,
+                    int nctas, int comm_mode, uint64_t shard_off, int comm_split) {
+  return ag_gemm_impl(c, stream, a_shard, B, C, gather_off, flags_off, epoch, M, N, K, ldc, ncomm, nctas, comm_mode,
+                      shard_off, comm_split, false, nullptr, nullptr, act);
 }
 // MXFP8 variant: payloads are e4m3 bytes; `sfa` is the tiled scale tensor of the GATHERED A (every rank must
 // hold all of it before the call, e.g. through an all-gather of the small scale tensors), `sfb` that of B.

@@ -9,6 +9,13 @@ namespace mt {
 
 enum GemmMode : int { MODE_PLAIN = 0, MODE_AG_GEMM = 1, MODE_GEMM_RS = 2 };
 
+// What the epilogue of a bf16 CTA-pair GEMM (plain, all-gather -> GEMM) does besides storing C.
+enum GemmEpi : int {
+  EPI_NONE = 0,
+  EPI_SILU = 1,    // aux = silu(C), C as rounded
+  EPI_DSILU = 2,   // C = C * silu'(aux), aux read, C as rounded
+};
+
 // TMA descriptors, one set per local rank (index 0 outside single-GPU emulation).
 struct GemmMaps {
   CUtensorMap a[MT_MAX_RANKS];   // A operand: [M, K] (AG_GEMM: the gathered buffer)
@@ -33,6 +40,8 @@ struct GemmArgs {
   int32_t comm_split;                  // AG_GEMM: comm CTAs that share one 128-row chunk
   int32_t ta, tb;                      // CTA pairs, bf16: the operand is stored [K, M] / [K, N] (ta: plain GEMM only,
                                        // tb: plain and GEMM_RS); its map then has boxes of 64 columns x 64 K rows
+  int32_t epi;                         // GemmEpi
+  void* aux[MT_MAX_RANKS];             // second output (EPI_SILU) or input (EPI_DSILU), laid out like C
   int32_t raster;                      // plain GEMM: row blocks per group of the tile order (<= 1: row-major)
   uint64_t shard_off;                  // AG_GEMM pull: heap offset of every rank's own rows
   uint64_t gather_off;                 // AG_GEMM: heap offset of the gathered A buffer [M, K]

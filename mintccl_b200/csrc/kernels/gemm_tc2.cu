@@ -93,6 +93,25 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatil
   return true;
 }
 
+// silu and its derivative on eight packed bf16, in fp32.  The exponential and the quotient are the fast forms (their
+// error is 1e-6, the result is rounded to 8 bits): with expf and an exact division the last tile's epilogue is longer
+// than what the torch pass costs.
+__device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+  return *(uint32_t*)&p;
+}
+__device__ __forceinline__ uint32_t silu2(uint32_t v) {
+  const float a = __uint_as_float(v << 16), b = __uint_as_float(v & 0xffff0000u);
+  return pack_bf16(a * sigmoid_fast(a), b * sigmoid_fast(b));
+}
+__device__ __forceinline__ uint32_t dsilu2(uint32_t d, uint32_t h) {
+  const float a = __uint_as_float(h << 16), b = __uint_as_float(h & 0xffff0000u);
+  const float sa = sigmoid_fast(a), sb = sigmoid_fast(b);
+  return pack_bf16(__uint_as_float(d << 16) * (sa * (1.f + a * (1.f - sa))),
+                   __uint_as_float(d & 0xffff0000u) * (sb * (1.f + b * (1.f - sb))));
+}
+
 // Tile order: fused_schedule.h with 256-row tiles (mb, jb count 256-row blocks).
 using Tile = MtTile;
 template <int MODE, int TILE_N>
@@ -334,6 +353,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       const bool rows_out = MODE != MODE_PLAIN || tc_.mb * BM2 + (int)cr * BMC < a.M;   // M % 256 == 128: last peer has none
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN;
       const uint32_t acc_empty0 = map_to_cta(smem_u32(&ctl->acc_empty[as]), 0);
+      // activation fused into the epilogue: aux has C's layout (the work overlaps the next tile's main loop)
+      constexpr bool kEpi = MODE != MODE_GEMM_RS && !FP8;
+      const int epi = kEpi ? a.epi : EPI_NONE;
+      uint8_t* aux = (uint8_t*)a.aux[lr] + (dst - (uint8_t*)a.c[lr]);
+      uint4 hv[8];
       // 4 rows per pass of 8 lanes x 16 bytes: full 128-byte lines
       // `nchunk` 16-byte pieces per row: 8 for a full block of 64 columns, 4 for the last half block of a 224 tile
       auto store_block = [&](int cb, int nchunk = 8) {
@@ -349,8 +373,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             w.x = (uint64_t)v.x | ((uint64_t)v.y << 32);
             w.y = (uint64_t)v.z | ((uint64_t)v.w << 32);
             store128_relaxed_sys(g, w);
+          } else if (kEpi && epi == EPI_DSILU) {
+            *(uint4*)g = make_uint4(dsilu2(v.x, hv[p].x), dsilu2(v.y, hv[p].y), dsilu2(v.z, hv[p].z), dsilu2(v.w, hv[p].w));
           } else {
             *(uint4*)g = v;
+            if (kEpi && epi == EPI_SILU)
+              *(uint4*)(aux + (uint64_t)rr * ld_bytes + cb * 128 + c16 * 16) = make_uint4(silu2(v.x), silu2(v.y), silu2(v.z), silu2(v.w));
           }
         }
       };
@@ -389,6 +417,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         for (int cb = 0; cb < (BN + 63) / 64; ++cb) {
           uint32_t r0[32], r1[32];
           const bool half = cb * 64 + 32 >= BN;   // only 32 columns left (224 = 3 x 64 + 32)
+          if (kEpi && epi == EPI_DSILU && rows_out) {
+#pragma unroll
+            for (int p = 0; p < 8; ++p)
+              if ((lane & 7) < (half ? 4 : 8))
+                hv[p] = *(const uint4*)(aux + (uint64_t)(p * 4 + (lane >> 3)) * ld_bytes + cb * 128 + (lane & 7) * 16);
+          }
           tmem_ld_32x32(taddr + cb * 64, r0);
           if (!half) tmem_ld_32x32(taddr + cb * 64 + 32, r1);
           tmem_ld_wait();

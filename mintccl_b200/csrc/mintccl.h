@@ -124,6 +124,11 @@ int mt_gemm_mxfp8(void* stream, const void* A, const void* sfa, const void* B, c
 // Operands stored transposed: A as [K, M] (ta), B as [K, N] (tb); CTA pairs only.
 int mt_gemm_t(void* stream, const void* A, const void* B, void* C, int M, int N, int K, int ta, int tb);
 int mt_gemm_uses_pair(int rows);
+// C = (A[M, K] * B[K, N]) * silu'(H), and all-gather -> GEMM that also stores act = silu(C) (CTA pairs only)
+int mt_gemm_dsilu(void* stream, const void* A, const void* B, const void* H, void* C, int M, int N, int K);
+int mt_ag_gemm_silu(MtComm* c, void* stream, const void* const* a_shard, const void* const* B, void* const* C, void* const* act,
+                    uint64_t gather_off, uint64_t flags_off, uint64_t epoch, int M, int N, int K, int ldc, int ncomm,
+                    int nctas, int comm_mode, uint64_t shard_off, int comm_split);
 int mt_gemm_rs_t(MtComm* c, void* stream, const void* const* A, const void* const* B, void* const* out,
                  uint64_t stage_off, uint64_t flags_off, uint64_t epoch, int M, int N, int K, int nred, int nctas);
 // Plain GEMMs with M % 256 == 0 run on CTA pairs (tcgen05 cta_group::2) when MINTCCL_GEMM_PAIR is not 0; a wait

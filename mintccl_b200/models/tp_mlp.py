@@ -3,9 +3,9 @@ projection, activations sharded over tokens between blocks) built on the fused k
 
     x_shard [T / n, H]  --all-gather -> GEMM-->  h [T, F / n]  --act-->  --GEMM -> reduce-scatter-->  y_shard [T / n, H]
 
-The forward pass is two kernel launches (``AllGatherGemm``, ``GemmReduceScatter``) plus the activation.
-The backward pass runs the transposed products through the same tcgen05 GEMM and the library's own
-collectives.  This is the "fuse the collectives with your own kernels" use case the reference names as its
+The forward pass is two kernel launches: ``AllGatherGemm``, whose epilogue also stores the activation, and
+``GemmReduceScatter``.  The backward pass runs the transposed products through the same tcgen05 GEMM (operands as they
+are stored, the derivative of the activation in the epilogue) and the library's own collectives.  This is the "fuse the collectives with your own kernels" use case the reference names as its
 purpose (README.md:5) but does not implement; the shapes of the benchmark are the Llama-3-8B MLP ones
 (tokens 8192, hidden 4096, ffn 14336, TP = 8).
 """
@@ -15,14 +15,13 @@ from typing import Optional
 
 import torch
 
-from ..ops.gemm import AllGatherGemm, GemmReduceScatter, gemm_t
+from ..ops.gemm import AllGatherGemm, GemmReduceScatter, gemm_dsilu, gemm_t
 
 
 class _MLPFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x_shard, w_up, w_down, mlp):
-        h = mlp.ag_gemm(x_shard, w_up)                       # [T, F/n]
-        a = torch.nn.functional.silu(h)
+        h, a = mlp.ag_gemm.call_silu(x_shard, w_up)          # [T, F/n], and silu of it
         y = mlp.gemm_rs(a, w_down)                           # [T/n, H]
         ctx.mlp = mlp
         ctx.save_for_backward(x_shard, w_up, w_down, h, a)
@@ -41,10 +40,8 @@ class _MLPFunction(torch.autograd.Function):
         if n > 1:
             x = x.clone()
             x[comm.rank * (T // n):(comm.rank + 1) * (T // n)].copy_(x_shard)
-        da = gemm_t(dy, w_down, tb=True)                     # [T, F/n] = dy @ w_down       (w_down: [H, F/n])
+        dh = gemm_dsilu(dy, w_down, h)                       # [T, F/n] = (dy @ w_down) * silu'(h)   (w_down: [H, F/n])
         dw_down = gemm_t(dy, a, ta=True, tb=True)            # [H, F/n] = dy^T @ a
-        sig = torch.sigmoid(h.float())
-        dh = (da.float() * (sig * (1 + h.float() * (1 - sig)))).to(torch.bfloat16)
         dw_up = gemm_t(dh, x, ta=True, tb=True)              # [F/n, H] = dh^T @ x
         dx_shard = mlp.gemm_rs_bwd.call_transposed(dh, w_up)      # reduce_scatter(dh @ w_up)    (w_up: [F/n, H])
         return dx_shard, dw_up, dw_down, None

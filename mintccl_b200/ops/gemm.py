@@ -64,6 +64,19 @@ def gemm_t(a: torch.Tensor, b: torch.Tensor, ta: bool = False, tb: bool = False)
     return out
 
 
+def gemm_dsilu(d: torch.Tensor, w: torch.Tensor, h: torch.Tensor) -> torch.Tensor:
+    """``(d[M, K] @ w[K, N]) * silu'(h)``: the gradient of a linear layer's input carried through the silu before it."""
+    for t, name in ((d, "d"), (w, "w"), (h, "h")):
+        _check(t, name)
+    if d.shape[1] != w.shape[0] or tuple(h.shape) != (d.shape[0], w.shape[1]):
+        raise ValueError("operand shapes do not match")
+    out = torch.empty_like(h)
+    stream = torch.cuda.current_stream(d.device).cuda_stream
+    if N.lib().mt_gemm_dsilu(stream, d.data_ptr(), w.data_ptr(), h.data_ptr(), out.data_ptr(), d.shape[0], w.shape[1], d.shape[1]) < 0:
+        raise RuntimeError(f"mt_gemm_dsilu: {N.last_error()}")
+    return out
+
+
 class _Fused:
     def __init__(self, comm):
         self.comm = comm
@@ -167,6 +180,19 @@ class AllGatherGemm(_Fused):
         return max(nc for nc in range(lo, hi + 1) if waves(nc) == best)
 
     def __call__(self, a_shard: TensorOrList, w: TensorOrList, out: Optional[TensorOrList] = None, nctas: int = 0):
+        return self._run(a_shard, w, out, nctas, None)
+
+    def call_silu(self, a_shard: TensorOrList, w: TensorOrList):
+        """``(h, silu(h))`` with ``h`` the product: the epilogue stores both."""
+        c = self.comm
+        ws = self._lists(w)
+        if c.world_size > 1 and (self.mode == 2 or not c.lib.mt_gemm_uses_pair(self.M // c.world_size)):
+            hs = self._run(a_shard, w, None, 0, None)     # single-CTA kernels: the activation is a pass of its own
+            return hs, ([torch.nn.functional.silu(h) for h in hs] if c.emulated else torch.nn.functional.silu(hs))
+        act = [torch.empty(self.M, self.N, device=t.device, dtype=torch.bfloat16) for t in ws]
+        return self._run(a_shard, w, None, 0, act), (act if c.emulated else act[0])
+
+    def _run(self, a_shard, w, out, nctas, act):
         c = self.comm
         a_s, ws = self._lists(a_shard), self._lists(w)
         if out is None:
@@ -184,10 +210,11 @@ class AllGatherGemm(_Fused):
                 raise ValueError("mode='pull' needs a_shard from the symmetric heap")
             shard_off = offs[0]
         self.epoch += 1
-        rc = c.lib.mt_ag_gemm(c._handle, c._stream(), N.ptr_array([t.data_ptr() for t in a_s]),
-                              N.ptr_array([t.data_ptr() for t in ws]), N.ptr_array([t.data_ptr() for t in outs]),
-                              self._off(self.gathered), self._off(self.flags), self.epoch, self.M, self.N, self.K,
-                              outs[0].stride(0), self.ncomm, nctas, self.mode, shard_off, self.split)
+        fn, extra = (c.lib.mt_ag_gemm, ()) if act is None else (c.lib.mt_ag_gemm_silu, (N.ptr_array([t.data_ptr() for t in act]),))
+        rc = fn(c._handle, c._stream(), N.ptr_array([t.data_ptr() for t in a_s]),
+                N.ptr_array([t.data_ptr() for t in ws]), N.ptr_array([t.data_ptr() for t in outs]), *extra,
+                self._off(self.gathered), self._off(self.flags), self.epoch, self.M, self.N, self.K,
+                outs[0].stride(0), self.ncomm, nctas, self.mode, shard_off, self.split)
         if rc < 0:
             raise RuntimeError(f"mt_ag_gemm: {N.last_error()}")
         return outs if c.emulated else outs[0]

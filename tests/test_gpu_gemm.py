@@ -209,3 +209,41 @@ def test_gemm_rs_with_a_transposed_weight(n, rows):
         w_.check()
         for x, y in zip(got, want):
             assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("n,T,F,K", [(1, 128, 256, 64), (1, 384, 1792, 128), (1, 8192, 1792, 256), (2, 512, 512, 128), (2, 256, 512, 128),
+                                     (4, 1024, 1792, 192)])
+def test_silu_in_the_epilogue(n, T, F, K):
+    """h is the same with and without the activation, and the activation is torch's silu of h up to one rounding of the
+    fp32 value (the fast exponential is 1e-6 off, which moves a result by one bf16 step at most)."""
+    from mintccl_b200.ops.gemm import AllGatherGemm
+    w_ = world(n)
+    plan = AllGatherGemm(w_, T, F, K, ncomm=4)
+    g = torch.Generator(device="cuda").manual_seed(T + F)
+    xs = [torch.randn(T // n, K, generator=g, device="cuda").to(torch.bfloat16) for _ in range(n)]
+    ws = [torch.randn(F, K, generator=g, device="cuda").to(torch.bfloat16) for _ in range(n)]
+    xs[0][0, :] = 100.0            # products far outside the range of the exponential
+    plain = [h.clone() for h in plan(xs, ws)]
+    hs, acts = plan.call_silu(xs, ws)
+    w_.check()
+    for h, a, p in zip(hs, acts, plain):
+        close(h, p.float(), K)
+        want = torch.nn.functional.silu(h.float())
+        assert bool(((a.float() - want).abs() <= 2 ** -8 * 1.001 * want.abs() + 1e-35).all())
+
+
+@pytest.mark.parametrize("shape", [(128, 256, 64), (384, 1792, 128), (8192, 1792, 256), (2048, 512, 448)])
+def test_silu_derivative_in_the_epilogue(shape):
+    from mintccl_b200.ops.gemm import gemm_dsilu, gemm_t
+    T, F, K = shape
+    g = torch.Generator(device="cuda").manual_seed(T + K)
+    d = torch.randn(T, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(K, F, generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    h = (torch.randn(T, F, generator=g, device="cuda") * 3).to(torch.bfloat16)
+    h[0, :8] = torch.tensor([-1e4, -90.0, -88.0, 0.0, 88.0, 90.0, 1e4, -20.0], device="cuda").to(torch.bfloat16)
+    got = gemm_dsilu(d, w, h)
+    da = gemm_t(d, w, tb=True).float()
+    sig = torch.sigmoid(h.float())
+    want = da * (sig * (1 + h.float() * (1 - sig)))
+    # one rounding; where 1 + h (1 - sig) cancels the fp32 factor itself is 1e-6 off
+    assert bool(((got.float() - want).abs() <= 2 ** -8 * 1.001 * want.abs() + 4e-6 * da.abs()).all())
