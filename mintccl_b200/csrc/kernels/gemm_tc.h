@@ -41,6 +41,7 @@ struct GemmArgs {
   int32_t ta, tb;                      // CTA pairs, bf16: the operand is stored [K, M] / [K, N] (ta: plain GEMM only,
                                        // tb: plain and GEMM_RS); its map then has boxes of 64 columns x 64 K rows
   int32_t epi;                         // GemmEpi
+  int32_t wide_out;                    // rows of C (and aux) start on 32-byte boundaries
   void* aux[MT_MAX_RANKS];             // second output (EPI_SILU) or input (EPI_DSILU), laid out like C
   int32_t raster;                      // plain GEMM: row blocks per group of the tile order (<= 1: row-major)
   uint64_t shard_off;                  // AG_GEMM pull: heap offset of every rank's own rows

@@ -51,7 +51,6 @@ namespace pair {
 
 constexpr int BMC = 128;   // A rows (and accumulator rows) per CTA
 constexpr int BM2 = 256;   // rows of the pair's tile
-constexpr int BN = 256;    // columns of the tile
 constexpr int BNC = 128;   // B rows staged by each CTA
 constexpr int STAGES = 6;
 constexpr int kThreads = 192;
@@ -93,13 +92,58 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatil
   return true;
 }
 
-// silu and its derivative on eight packed bf16, in fp32.  The exponential and the quotient are the fast forms (their
+// 32 bf16 of one row (64 bytes) in two 32-byte accesses, or in four of 16 bytes where the matrix is only aligned to that.
+__device__ __forceinline__ void store_row64(uint8_t* p, const uint32_t* v, bool wide) {
+  if (wide) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p + j * 32), "r"(v[8 * j]), "r"(v[8 * j + 1]),
+                   "r"(v[8 * j + 2]), "r"(v[8 * j + 3]), "r"(v[8 * j + 4]), "r"(v[8 * j + 5]), "r"(v[8 * j + 6]), "r"(v[8 * j + 7])
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *(uint4*)(p + j * 16) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  }
+}
+__device__ __forceinline__ void load_row64(const uint8_t* p, uint32_t* v, bool wide) {
+  if (wide) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(v[8 * j]), "=r"(v[8 * j + 1]), "=r"(v[8 * j + 2]), "=r"(v[8 * j + 3]), "=r"(v[8 * j + 4]),
+                     "=r"(v[8 * j + 5]), "=r"(v[8 * j + 6]), "=r"(v[8 * j + 7])
+                   : "l"(p + j * 32));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint4 t = *(const uint4*)(p + j * 16);
+      v[4 * j] = t.x;
+      v[4 * j + 1] = t.y;
+      v[4 * j + 2] = t.z;
+      v[4 * j + 3] = t.w;
+    }
+  }
+}
+
+// silu and its derivative on two packed bf16, in fp32.  The exponential and the quotient are the fast forms (their
 // error is 1e-6, the result is rounded to 8 bits): with expf and an exact division the last tile's epilogue is longer
 // than what the torch pass costs.
 __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
   return *(uint32_t*)&p;
+}
+// 64 accumulator columns of this lane's row as packed bf16.
+__device__ __forceinline__ void tmem_ld_pack64(uint32_t taddr, uint32_t* v) {
+  uint32_t r0[32], r1[32];
+  tmem_ld_32x32(taddr, r0);
+  tmem_ld_32x32(taddr + 32, r1);
+  tmem_ld_wait();
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    v[j] = pack_bf16(__uint_as_float(r0[2 * j]), __uint_as_float(r0[2 * j + 1]));
+    v[16 + j] = pack_bf16(__uint_as_float(r1[2 * j]), __uint_as_float(r1[2 * j + 1]));
+  }
 }
 __device__ __forceinline__ uint32_t silu2(uint32_t v) {
   const float a = __uint_as_float(v << 16), b = __uint_as_float(v & 0xffff0000u);
@@ -353,104 +397,101 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       const bool rows_out = MODE != MODE_PLAIN || tc_.mb * BM2 + (int)cr * BMC < a.M;   // M % 256 == 128: last peer has none
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN;
       const uint32_t acc_empty0 = map_to_cta(smem_u32(&ctl->acc_empty[as]), 0);
-      // activation fused into the epilogue: aux has C's layout (the work overlaps the next tile's main loop)
-      constexpr bool kEpi = MODE != MODE_GEMM_RS && !FP8;
-      const int epi = kEpi ? a.epi : EPI_NONE;
-      uint8_t* aux = (uint8_t*)a.aux[lr] + (dst - (uint8_t*)a.c[lr]);
-      uint4 hv[8];
-      // 4 rows per pass of 8 lanes x 16 bytes: full 128-byte lines
-      // `nchunk` 16-byte pieces per row: 8 for a full block of 64 columns, 4 for the last half block of a 224 tile
-      auto store_block = [&](int cb, int nchunk = 8) {
-        if (!rows_out) return;
+      if constexpr (MODE == MODE_GEMM_RS) {
+        // Partial tiles go to a peer: whole 128-byte lines per store (a transpose through shared memory, 4 rows per pass
+        // of 8 lanes x 16 bytes), so that NVLink carries full packets.
+        auto store_block = [&](int cb) {
 #pragma unroll
-        for (int p = 0; p < 8; ++p) {
-          const int rr = p * 4 + (lane >> 3), c16 = lane & 7;
-          if (c16 >= nchunk) continue;
-          const uint4 v = *(const uint4*)(stg + rr * EPI_PITCH + c16 * 16);
-          uint8_t* g = dst + (uint64_t)rr * ld_bytes + cb * 128 + c16 * 16;
-          if (MODE == MODE_GEMM_RS) {
+          for (int p = 0; p < 8; ++p) {
+            const int rr = p * 4 + (lane >> 3), c16 = lane & 7;
+            const uint4 v = *(const uint4*)(stg + rr * EPI_PITCH + c16 * 16);
             u128 w;
             w.x = (uint64_t)v.x | ((uint64_t)v.y << 32);
             w.y = (uint64_t)v.z | ((uint64_t)v.w << 32);
-            store128_relaxed_sys(g, w);
-          } else if (kEpi && epi == EPI_DSILU) {
-            *(uint4*)g = make_uint4(dsilu2(v.x, hv[p].x), dsilu2(v.y, hv[p].y), dsilu2(v.z, hv[p].z), dsilu2(v.w, hv[p].w));
-          } else {
-            *(uint4*)g = v;
-            if (kEpi && epi == EPI_SILU)
-              *(uint4*)(aux + (uint64_t)rr * ld_bytes + cb * 128 + c16 * 16) = make_uint4(silu2(v.x), silu2(v.y), silu2(v.z), silu2(v.w));
+            store128_relaxed_sys(dst + (uint64_t)rr * ld_bytes + cb * 128 + c16 * 16, w);
           }
-        }
-      };
-      if constexpr (FP8) {
-        // single accumulator: drain it into registers (packed bf16) first and hand it back, then store
-        uint32_t pk[BN / 2];
-#pragma unroll
-        for (int cb = 0; cb < BN / 64; ++cb) {
-          uint32_t r0[32], r1[32];
-          tmem_ld_32x32(taddr + cb * 64, r0);
-          tmem_ld_32x32(taddr + cb * 64 + 32, r1);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            __nv_bfloat162 p0 = __floats2bfloat162_rn(__uint_as_float(r0[2 * j]), __uint_as_float(r0[2 * j + 1]));
-            __nv_bfloat162 p1 = __floats2bfloat162_rn(__uint_as_float(r1[2 * j]), __uint_as_float(r1[2 * j + 1]));
-            pk[cb * 32 + j] = *(uint32_t*)&p0;
-            pk[cb * 32 + 16 + j] = *(uint32_t*)&p1;
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(acc_empty0);
-#pragma unroll
-        for (int cb = 0; cb < BN / 64; ++cb) {
+        };
+        uint32_t pk[FP8 ? BN / 2 : 32];
+        auto stage_block = [&](int cb, const uint32_t* v) {
           uint4* row = (uint4*)(stg + lane * EPI_PITCH);
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            row[j] = make_uint4(pk[cb * 32 + 4 * j], pk[cb * 32 + 4 * j + 1], pk[cb * 32 + 4 * j + 2], pk[cb * 32 + 4 * j + 3]);
+          for (int j = 0; j < 8; ++j) row[j] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
           __syncwarp();
           store_block(cb);
           __syncwarp();
+        };
+        if constexpr (FP8) {
+          // single accumulator: drain it into registers (packed bf16) first and hand it back, then store
+#pragma unroll
+          for (int cb = 0; cb < BN / 64; ++cb) tmem_ld_pack64(taddr + cb * 64, pk + cb * 32);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(acc_empty0);
+#pragma unroll
+          for (int cb = 0; cb < BN / 64; ++cb) stage_block(cb, pk + cb * 32);
+        } else {
+#pragma unroll 1
+          for (int cb = 0; cb < BN / 64; ++cb) {
+            tmem_ld_pack64(taddr + cb * 64, pk);
+            stage_block(cb, pk);
+          }
+          // accumulator drained: hand it back to the leader's MMA thread
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(acc_empty0);
         }
       } else {
+        // Local output: every lane keeps the row it got from TMEM and stores it in whole 32-byte sectors.  The tensor
+        // cores read the operands, and TMA writes them, at the full rate of the shared memory (64 KiB per 512 cycles and
+        // k-block), so an epilogue that transposes through shared memory takes its cycles from the main loop; it also took
+        // 2 us at the end of a small problem, where nothing hides it.
+        uint8_t* row = dst + (uint64_t)lane * ld_bytes;
+        // activation fused into the epilogue: aux has C's layout (the work overlaps the next tile's main loop)
+        const int epi = FP8 ? EPI_NONE : a.epi;
+        uint8_t* aux = (uint8_t*)a.aux[lr] + (row - (uint8_t*)a.c[lr]);
+        const bool wide = a.wide_out != 0;
+        auto store32 = [&](int c32, const uint32_t* v) {   // 32 columns: 64 bytes
+          store_row64(row + c32 * 64, v, wide);
+        };
+        if constexpr (FP8) {
+          uint32_t pk[BN / 2];
+#pragma unroll
+          for (int cb = 0; cb < BN / 64; ++cb) tmem_ld_pack64(taddr + cb * 64, pk + cb * 32);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(acc_empty0);
+          if (rows_out) {
+#pragma unroll
+            for (int c = 0; c < BN / 32; ++c) store32(c, pk + c * 16);
+          }
+        } else {
 #pragma unroll 1
-        for (int cb = 0; cb < (BN + 63) / 64; ++cb) {
-          uint32_t r0[32], r1[32];
-          const bool half = cb * 64 + 32 >= BN;   // only 32 columns left (224 = 3 x 64 + 32)
-          if (kEpi && epi == EPI_DSILU && rows_out) {
+          for (int c = 0; c < BN / 32; ++c) {
+            uint32_t r[32], v[16], h[16];
+            if (epi == EPI_DSILU && rows_out) load_row64(aux + c * 64, h, wide);
+            tmem_ld_32x32(taddr + c * 32, r);
+            tmem_ld_wait();
+            if (c == BN / 32 - 1) {
+              // accumulator drained: hand it back to the leader's MMA thread
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster(acc_empty0);
+            }
 #pragma unroll
-            for (int p = 0; p < 8; ++p)
-              if ((lane & 7) < (half ? 4 : 8))
-                hv[p] = *(const uint4*)(aux + (uint64_t)(p * 4 + (lane >> 3)) * ld_bytes + cb * 128 + (lane & 7) * 16);
-          }
-          tmem_ld_32x32(taddr + cb * 64, r0);
-          if (!half) tmem_ld_32x32(taddr + cb * 64 + 32, r1);
-          tmem_ld_wait();
-          uint4* row = (uint4*)(stg + lane * EPI_PITCH);
+            for (int j = 0; j < 16; ++j) v[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+            if (!rows_out) continue;
+            if (epi == EPI_DSILU) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            __nv_bfloat162 p0 = __floats2bfloat162_rn(__uint_as_float(r0[8 * j + 0]), __uint_as_float(r0[8 * j + 1]));
-            __nv_bfloat162 p1 = __floats2bfloat162_rn(__uint_as_float(r0[8 * j + 2]), __uint_as_float(r0[8 * j + 3]));
-            __nv_bfloat162 p2 = __floats2bfloat162_rn(__uint_as_float(r0[8 * j + 4]), __uint_as_float(r0[8 * j + 5]));
-            __nv_bfloat162 p3 = __floats2bfloat162_rn(__uint_as_float(r0[8 * j + 6]), __uint_as_float(r0[8 * j + 7]));
-            row[j] = make_uint4(*(uint32_t*)&p0, *(uint32_t*)&p1, *(uint32_t*)&p2, *(uint32_t*)&p3);
-          }
+              for (int j = 0; j < 16; ++j) v[j] = dsilu2(v[j], h[j]);
+            }
+            store32(c, v);
+            if (epi == EPI_SILU) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            __nv_bfloat162 p0 = __floats2bfloat162_rn(__uint_as_float(r1[8 * j + 0]), __uint_as_float(r1[8 * j + 1]));
-            __nv_bfloat162 p1 = __floats2bfloat162_rn(__uint_as_float(r1[8 * j + 2]), __uint_as_float(r1[8 * j + 3]));
-            __nv_bfloat162 p2 = __floats2bfloat162_rn(__uint_as_float(r1[8 * j + 4]), __uint_as_float(r1[8 * j + 5]));
-            __nv_bfloat162 p3 = __floats2bfloat162_rn(__uint_as_float(r1[8 * j + 6]), __uint_as_float(r1[8 * j + 7]));
-            row[4 + j] = make_uint4(*(uint32_t*)&p0, *(uint32_t*)&p1, *(uint32_t*)&p2, *(uint32_t*)&p3);
+              for (int j = 0; j < 16; ++j) v[j] = silu2(v[j]);
+              store_row64(aux + c * 64, v, wide);
+            }
           }
-          __syncwarp();
-          store_block(cb, half ? 4 : 8);
-          __syncwarp();
         }
-        // accumulator drained: hand it back to the leader's MMA thread
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(acc_empty0);
       }
       if (MODE == MODE_GEMM_RS) {
         // count this warp's quarter of the partial tile on the owner (release: the stores above come first)
@@ -562,6 +603,9 @@ cudaError_t launch_gemm_pair(int mode, const GemmMaps& maps, const PairSfMaps& s
   GemmMaps m = maps;
   PairSfMaps sm = sf;
   GemmArgs args = a;
+  uint64_t mis = (uint64_t)a.ldc * 2;
+  for (int lr = 0; lr < nlocal; ++lr) mis |= (uint64_t)(uintptr_t)a.c[lr] | (uint64_t)(uintptr_t)a.aux[lr];
+  args.wide_out = (mis & 31) == 0;
   void* p[] = {(void*)&m, (void*)&sm, (void*)&args};
   count_launch();
   const dim3 grid(2 * nclusters + extra, nlocal);
