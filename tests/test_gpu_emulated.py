@@ -624,3 +624,22 @@ def test_reduce_with_a_summing_root(n, numel, algo="direct2"):
             for r in range(n):
                 if r != root:
                     assert bool((outs[r] == -7.0).all())         # only the root's output is written
+
+
+@pytest.mark.parametrize("algo", ["direct", "pull", "bulk"])
+@pytest.mark.parametrize("nbytes", [1, 15, 17, 31, 47, 48, 49, 2047, 8193, 100_003])
+def test_allgather_of_rows_off_the_16_byte_grid(algo, nbytes):
+    """Rows whose size is no multiple of 16 and contributions that start anywhere: every pair of offsets of source and
+    destination, sizes around the vector, the warp's chunk and the CTA's slice.  Bytes outside the rows stay as they are."""
+    n = 4
+    w = world(n)
+    for start in (0, 1, 8, 13):
+        g = torch.Generator(device="cuda").manual_seed(nbytes + start)
+        src = [torch.randint(0, 256, (nbytes + start,), generator=g, device="cuda", dtype=torch.uint8)[start:] for _ in range(n)]
+        pads = [torch.full((n * nbytes + 64,), 7, device="cuda", dtype=torch.uint8) for _ in range(n)]
+        bufs = [p[32 + start:32 + start + n * nbytes].view(n, nbytes) for p in pads]
+        w.allgather(bufs, inp=src, algo=algo)
+        w.check()
+        for p, b in zip(pads, bufs):
+            assert torch.equal(b, torch.stack(src))
+            assert bool((p[:32 + start] == 7).all()) and bool((p[32 + start + n * nbytes:] == 7).all())
