@@ -643,3 +643,33 @@ def test_allgather_of_rows_off_the_16_byte_grid(algo, nbytes):
         for p, b in zip(pads, bufs):
             assert torch.equal(b, torch.stack(src))
             assert bool((p[:32 + start] == 7).all()) and bool((p[32 + start + n * nbytes:] == 7).all())
+
+
+@pytest.mark.parametrize("n", [2, 3, 4, 8])
+@pytest.mark.parametrize("blocks", [1, 5, 255, 4097])
+def test_mxfp8_sum_gives_the_bytes_of_the_oracle(n, blocks):
+    """Blocks per rank and CTA around the two-lane pairs and the block size of the kernel, in place and not.  The
+    dequantised terms are exact in fp32 and are added in rank order, so the oracle gives the same bytes."""
+    from mintccl_b200.ops import mxfp8 as mx
+    w = world(n)
+    numel = blocks * 32
+    q = [mx.quantize_mxfp8(x * 10.0 ** r) for r, x in enumerate(rand(n, numel, torch.float32, seed0=blocks))]
+    total = torch.zeros(numel, device="cuda")
+    for d, s in q:
+        total = total + mx.dequantize_mxfp8(d, s)
+    wd, ws = mx._torch_quantize(total)
+    data, scale = w.symm_empty(numel, torch.uint8), w.symm_empty(blocks, torch.uint8)
+    od, os_ = w.symm_empty(numel, torch.uint8), w.symm_empty(blocks, torch.uint8)
+    try:
+        for inplace in (False, True):
+            for r in range(n):
+                data[r].copy_(q[r][0])
+                scale[r].copy_(q[r][1])
+            mx.allreduce_mxfp8(w, data, scale, *(() if inplace else (od, os_)))
+            w.check()
+            for r in range(n):
+                assert torch.equal((scale if inplace else os_)[r], ws)
+                assert torch.equal((data if inplace else od)[r], wd)
+    finally:
+        for t in (data, scale, od, os_):
+            w.symm_free(t)
