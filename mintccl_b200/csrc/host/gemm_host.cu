@@ -477,11 +477,9 @@ int mt_gemm_rs_mxfp8(MtComm* c, void* stream, const void* const* A, const void* 
 int mt_mxfp8_quantize(void* stream, int dtype, const void* x, void* data, void* scale, uint64_t nelems) {
   if (nelems % 32) return fail("MXFP8 tensors hold whole blocks of 32 elements");
   if (dtype < 0 || dtype > 2) return fail("MXFP8 quantisation takes fp32, fp16 and bf16");
-  if (((uintptr_t)x & 15) || ((uintptr_t)data & 7)) return fail("MXFP8 quantisation needs a 16-byte aligned input");
+  if (((uintptr_t)x | (uintptr_t)data) & 15) return fail("MXFP8 quantisation needs 16-byte aligned buffers");
   if (nelems == 0) return 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  cudaError_t e = mt::launch_mx_quant(dtype, x, data, scale, nelems, sm_count(dev), (cudaStream_t)stream);
+  cudaError_t e = mt::launch_mx_quant(dtype, x, data, scale, nelems, (cudaStream_t)stream);
   if (e != cudaSuccess) return fail(std::string("mxfp8 quantise launch: ") + cudaGetErrorString(e));
   return 0;
 }

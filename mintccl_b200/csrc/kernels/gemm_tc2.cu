@@ -336,7 +336,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           // descriptor addresses are in units of 16 bytes and stay below 2^14: no carry into the other fields
           const uint64_t da = da0 + s * (A_BYTES >> 4), db = db0 + s * (B_PITCH >> 4);
           if (FP8) {
-            const uint32_t tsfa = tmem_base + 256, tsfb = tmem_base + 260;
+            const uint32_t tsfa = tmem_base + 256 + s * 16, tsfb = tsfa + 4;
             const uint8_t* sf = sSF + s * SF_STAGE_BYTES;
             tmem_cp_sf_pair(tsfa, make_smem_desc_sf(sf));
             tmem_cp_sf_pair(tsfb, make_smem_desc_sf(sf + 512));

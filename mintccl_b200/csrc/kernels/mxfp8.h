@@ -16,6 +16,6 @@ struct Mxfp8Args {
 };
 cudaError_t launch_mxfp8(const MtDevComm* comms, const Mxfp8Args& a, int nctas, int nlocal, cudaStream_t s);
 // mxfp8_quant.cu: encoding (nelems a multiple of 32, x 16-byte aligned) and scale reordering (kq = K / 128 words a row)
-cudaError_t launch_mx_quant(int dtype, const void* x, void* data, void* scale, uint64_t nelems, int sms, cudaStream_t s);
+cudaError_t launch_mx_quant(int dtype, const void* x, void* data, void* scale, uint64_t nelems, cudaStream_t s);
 cudaError_t launch_mx_tile(const void* in, void* out, uint32_t row_blocks, uint32_t kq, cudaStream_t s);
 }  // namespace mt

@@ -13,32 +13,36 @@
 
 namespace mt {
 
-constexpr int kQuantThreads = 256, kQuantUnroll = 4;
+constexpr int kQuantThreads = 256, kQuantUnroll = 2;
 
-// Eight consecutive elements as fp32.
-template <class T>
-struct Load8 {
-  static constexpr int kBytes = 16;
-  u128 v;
-  __device__ __forceinline__ void load(const uint8_t* p) { v = load128_stream(p); }
-  __device__ __forceinline__ void get(float* f) const {
-    T::unpack(v.x, f);
-    T::unpack(v.y, f + 4);
-  }
-};
-template <>
-struct Load8<F32> {
-  static constexpr int kBytes = 32;
-  u128 a, b;
+__device__ __forceinline__ void load256_stream(const uint8_t* p, uint32_t* v) {
+  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "l"(p));
+}
+// Half a block, 16 consecutive elements, as fp32.  WIDE: 32-byte loads (the input starts on a 32-byte boundary).
+template <class T, bool WIDE>
+struct Load16 {
+  static constexpr int kWords = 16 * (int)sizeof(typename T::elem) / 4;
+  uint32_t v[kWords];
   __device__ __forceinline__ void load(const uint8_t* p) {
-    a = load128_stream(p);
-    b = load128_stream(p + 16);
+    if constexpr (WIDE) {
+#pragma unroll
+      for (int i = 0; i < kWords / 8; ++i) load256_stream(p + 32 * i, v + 8 * i);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kWords / 4; ++i) {
+        const u128 t = load128_stream(p + 16 * i);
+        v[4 * i] = (uint32_t)t.x;
+        v[4 * i + 1] = (uint32_t)(t.x >> 32);
+        v[4 * i + 2] = (uint32_t)t.y;
+        v[4 * i + 3] = (uint32_t)(t.y >> 32);
+      }
+    }
   }
   __device__ __forceinline__ void get(float* f) const {
-    F32::unpack(a.x, f);
-    F32::unpack(a.y, f + 2);
-    F32::unpack(b.x, f + 4);
-    F32::unpack(b.y, f + 6);
+#pragma unroll
+    for (int i = 0; i < kWords / 2; ++i) T::unpack((uint64_t)v[2 * i] | ((uint64_t)v[2 * i + 1] << 32), f + i * T::kPer64);
   }
 };
 
@@ -48,83 +52,99 @@ __device__ __forceinline__ uint8_t e4m3_nosat(float q) {
   return float_to_e4m3(q);
 }
 
-// Bound by HBM: 3 bytes and a bit per bf16 element.  Four lanes share a block of 32 (8 elements each: 16-byte loads,
-// 8-byte stores, two shuffles for the block maximum), four groups per thread are in flight; the maximum is taken on
-// the bit patterns, where NaN is larger than everything, as amax has it.  The chain of torch kernels this replaces
-// made about a dozen passes over fp32 copies.  A linear layer of 8192 x 4096 -> 1792 (quantise, tile, GEMM) went from
-// 640 to 97 us with the two kernels of this file; the GEMM is 65 of them.
-template <class T>
+// Bound by HBM: 3 bytes and a bit per bf16 element; 8192 x 4096 takes 18.5 us on fixed buffers (5.4 TB/s).  Two lanes share a block of 32:
+// 32-byte loads, 16-byte stores, one shuffle for the block maximum.  (Four lanes with 16-byte loads and 8-byte stores
+// took 22 - 25 us whatever the unrolling and the grid.)  The maximum is taken on the bit patterns, where NaN is larger
+// than everything, as amax has it.  The chain of torch kernels this replaces made about a dozen passes over fp32
+// copies: a linear layer of 8192 x 4096 -> 1792 (quantise, tile, GEMM) took 640 us.
+template <class T, bool WIDE>
 __global__ void __launch_bounds__(kQuantThreads) mx_quant_kernel(const uint8_t* __restrict__ x, uint8_t* __restrict__ data,
-                                                                 uint8_t* __restrict__ scale, uint64_t ngroups) {
-  constexpr uint64_t kChunk = (uint64_t)kQuantThreads * kQuantUnroll;
-  for (uint64_t base = (uint64_t)blockIdx.x * kChunk; base < ngroups; base += (uint64_t)gridDim.x * kChunk) {
-    Load8<T> in[kQuantUnroll];
+                                                                 uint8_t* __restrict__ scale, uint64_t nhalves) {
+  constexpr int kBytes = 16 * (int)sizeof(typename T::elem);
+  const uint64_t base = (uint64_t)blockIdx.x * (kQuantThreads * kQuantUnroll) + threadIdx.x;
+  Load16<T, WIDE> in[kQuantUnroll];
 #pragma unroll
-    for (int u = 0; u < kQuantUnroll; ++u) {
-      const uint64_t g = base + u * kQuantThreads + threadIdx.x;
-      if (g < ngroups) in[u].load(x + g * Load8<T>::kBytes);
+  for (int u = 0; u < kQuantUnroll; ++u) {
+    const uint64_t g = base + u * kQuantThreads;
+    if (g < nhalves) in[u].load(x + g * kBytes);
+  }
+#pragma unroll
+  for (int u = 0; u < kQuantUnroll; ++u) {
+    // nhalves is even: the two lanes of a block are in or out together
+    const uint64_t g = base + u * kQuantThreads;
+    const bool live = g < nhalves;
+    float f[16];
+    uint32_t m = 0;
+    if (live) {
+      in[u].get(f);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) m = max(m, __float_as_uint(f[i]) & 0x7fffffffu);
     }
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    if (!live) continue;
+    // smallest power of two 2^(e - 127) with amax <= 448 * 2^(e - 127): from the exponent, one more past 1.75 * 2^k
+    uint32_t e = 127 - 8;
+    if (m >= 0x7f800000u) e = ue8m0_for_amax(__uint_as_float(m));
+    else if (m != 0) e = (uint32_t)max((int)(m >> 23) - 8 + ((m & 0x7fffffu) > 0x600000u ? 1 : 0), 1);
+    const float inv = __uint_as_float(e == 254u ? 0x00400000u : (254u - e) << 23);   // 2^(127 - e): exact
+    uint32_t w[4] = {0, 0, 0, 0};
+    if (m < 0x7f800000u) {   // every quotient is at most 448: nothing saturates
 #pragma unroll
-    for (int u = 0; u < kQuantUnroll; ++u) {
-      // ngroups is a multiple of 4: the four lanes of a block are in or out together
-      const uint64_t g = base + u * kQuantThreads + threadIdx.x;
-      const bool live = g < ngroups;
-      float f[8];
-      uint32_t m = 0;
-      if (live) {
-        in[u].get(f);
+      for (int i = 0; i < 8; ++i)
+        w[i >> 1] |= (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(f[2 * i] * inv, f[2 * i + 1] * inv), __NV_SATFINITE, __NV_E4M3)
+                     << (16 * (i & 1));
+    } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) m = max(m, __float_as_uint(f[i]) & 0x7fffffffu);
-      }
-      m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
-      m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
-      if (!live) continue;
-      const uint32_t e = ue8m0_for_amax(__uint_as_float(m));
-      const float inv = __uint_as_float(e == 254u ? 0x00400000u : (254u - e) << 23);   // 2^(127 - e): exact
-      uint64_t w = 0;
-      if (m < 0x7f800000u) {   // every quotient is at most 448: nothing saturates
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          w |= (uint64_t)__nv_cvt_float2_to_fp8x2(make_float2(f[2 * i] * inv, f[2 * i + 1] * inv), __NV_SATFINITE, __NV_E4M3)
-               << (16 * i);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) w |= (uint64_t)e4m3_nosat(f[i] * inv) << (8 * i);
-      }
-      *reinterpret_cast<uint64_t*>(data + g * 8) = w;
-      if ((threadIdx.x & 3) == 0) scale[g >> 2] = (uint8_t)e;
+      for (int i = 0; i < 16; ++i) w[i >> 2] |= (uint32_t)e4m3_nosat(f[i] * inv) << (8 * (i & 3));
     }
+    *reinterpret_cast<uint4*>(data + g * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+    if ((threadIdx.x & 1) == 0) scale[g >> 1] = (uint8_t)e;
   }
 }
 
 // Scales [rows, kq] of 4-byte words (four blocks along K) -> [rows / 128][kq][32][4] words: word (r % 32, (r % 128) / 32)
-// of an atom.  One CTA takes 128 rows x 32 words through shared memory, so that both sides are whole lines.
+// of an atom.  One CTA takes 128 rows x 8 words through shared memory: whole sectors on the reading side, whole lines on
+// the writing side, all loads of a thread in flight, and enough CTAs (8192 x 4096 has 256) that the one round trip is all
+// that is left.
+constexpr int kTileWords = 8;
 __global__ void __launch_bounds__(256) mx_tile_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t kq) {
-  __shared__ uint32_t s[128][33];
-  const uint32_t R = blockIdx.y, k0 = blockIdx.x * 32;
-  const uint32_t nk = min(32u, kq - k0);
-  for (uint32_t i = threadIdx.x; i < 128 * 32; i += 256) {
-    const uint32_t r = i >> 5, k = i & 31;
-    if (k < nk) s[r][k] = in[((uint64_t)R * 128 + r) * kq + k0 + k];
+  __shared__ uint32_t s[128][kTileWords + 1];
+  const uint32_t R = blockIdx.y, k0 = blockIdx.x * kTileWords;
+  const uint32_t nk = min((uint32_t)kTileWords, kq - k0);
+  uint32_t v[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t r = j * 32 + (threadIdx.x >> 3), k = threadIdx.x & 7;
+    if (k < nk) v[j] = in[((uint64_t)R * 128 + r) * kq + k0 + k];
   }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s[j * 32 + (threadIdx.x >> 3)][threadIdx.x & 7] = v[j];
   __syncthreads();
   uint32_t* o = out + ((uint64_t)R * kq + k0) * 128;
-  for (uint32_t i = threadIdx.x; i < nk * 128; i += 256) {
-    const uint32_t w = i & 127;   // word of the atom
-    o[i] = s[(w & 3) * 32 + (w >> 2)][i >> 7];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t i = j * 256 + threadIdx.x, w = i & 127;   // word of the atom
+    if (i < nk * 128) o[i] = s[(w & 3) * 32 + (w >> 2)][i >> 7];
   }
 }
 
-cudaError_t launch_mx_quant(int dtype, const void* x, void* data, void* scale, uint64_t nelems, int sms, cudaStream_t s) {
-  const uint64_t groups = nelems / 8, chunk = (uint64_t)kQuantThreads * kQuantUnroll;
-  uint64_t grid = (groups + chunk - 1) / chunk;
-  if (grid > (uint64_t)sms * 8) grid = (uint64_t)sms * 8;
-  const uint8_t* p = (const uint8_t*)x;
+template <class T>
+static void go_quant(const void* x, void* data, void* scale, uint64_t nelems, cudaStream_t s) {
+  const uint64_t halves = nelems / 16, chunk = (uint64_t)kQuantThreads * kQuantUnroll;
+  const unsigned grid = (unsigned)((halves + chunk - 1) / chunk);
+  if (((uintptr_t)x & 31) == 0)
+    mx_quant_kernel<T, true><<<grid, kQuantThreads, 0, s>>>((const uint8_t*)x, (uint8_t*)data, (uint8_t*)scale, halves);
+  else
+    mx_quant_kernel<T, false><<<grid, kQuantThreads, 0, s>>>((const uint8_t*)x, (uint8_t*)data, (uint8_t*)scale, halves);
+}
+
+cudaError_t launch_mx_quant(int dtype, const void* x, void* data, void* scale, uint64_t nelems, cudaStream_t s) {
+  if (nelems / 16 / (kQuantThreads * kQuantUnroll) >= 0x7fffffffull) return cudaErrorInvalidValue;
   count_launch();
   switch (dtype) {
-    case DT_F32: mx_quant_kernel<F32><<<(unsigned)grid, kQuantThreads, 0, s>>>(p, (uint8_t*)data, (uint8_t*)scale, groups); break;
-    case DT_F16: mx_quant_kernel<F16><<<(unsigned)grid, kQuantThreads, 0, s>>>(p, (uint8_t*)data, (uint8_t*)scale, groups); break;
-    case DT_BF16: mx_quant_kernel<BF16><<<(unsigned)grid, kQuantThreads, 0, s>>>(p, (uint8_t*)data, (uint8_t*)scale, groups); break;
+    case DT_F32: go_quant<F32>(x, data, scale, nelems, s); break;
+    case DT_F16: go_quant<F16>(x, data, scale, nelems, s); break;
+    case DT_BF16: go_quant<BF16>(x, data, scale, nelems, s); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -132,7 +152,7 @@ cudaError_t launch_mx_quant(int dtype, const void* x, void* data, void* scale, u
 
 cudaError_t launch_mx_tile(const void* in, void* out, uint32_t row_blocks, uint32_t kq, cudaStream_t s) {
   count_launch();
-  mx_tile_kernel<<<dim3((kq + 31) / 32, row_blocks), 256, 0, s>>>((const uint32_t*)in, (uint32_t*)out, kq);
+  mx_tile_kernel<<<dim3((kq + kTileWords - 1) / kTileWords, row_blocks), 256, 0, s>>>((const uint32_t*)in, (uint32_t*)out, kq);
   return cudaGetLastError();
 }
 
