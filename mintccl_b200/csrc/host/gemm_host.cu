@@ -109,35 +109,62 @@ static int raster_for(int /*M*/, int N, int K, int elem_bytes) {
   return b_bytes > 48e6 ? 16 : 1;
 }
 
-// GEMMs run on CTA pairs (one 256 x 256 tile per cluster of two CTAs, gemm_tc2.cu) when the rows (of the
-// problem for the plain GEMM, of one rank for the fused kernels) are a multiple of 256; otherwise, and with
-// MINTCCL_GEMM_PAIR=0, on the single-CTA kernels of gemm_tc.cu.
+// GEMMs run on CTA pairs (gemm_tc2.cu); the fused kernels when a rank's rows are a multiple of 256, plain ones always (a last
+// block of 128 rows leaves its peer CTA idle).  MINTCCL_GEMM_PAIR=0: the single-CTA kernels of gemm_tc.cu.
 static int g_pair_mode = -1;
-static bool use_pair(int M) {
+static bool pair_on() {
   if (g_pair_mode < 0) {
     const char* e = getenv("MINTCCL_GEMM_PAIR");
     g_pair_mode = e ? atoi(e) : kPairDefault;
   }
-  return g_pair_mode != 0 && M % 256 == 0;
+  return g_pair_mode != 0;
 }
+static bool use_pair(int M) { return pair_on() && M % 256 == 0; }
 
 // Tile width of a bf16 pair GEMM over `row_tiles` 256-row blocks on `nclusters` clusters: 224 columns when N
-// allows it and the waves of narrower tiles add up to less work than the waves of 256-column tiles
-// (MINTCCL_GEMM_BN=256 / 224 forces one).
-static int pick_bn(int row_tiles, int N, int nclusters, bool fp8) {
+// allows it and the waves of narrower tiles add up to less work than the waves of 256-column tiles.
+static int pick_wide(int row_tiles, int N, int nclusters, bool fp8) {
   if (fp8 || N % 224 || nclusters < 1) return 256;
-  if (const char* e = getenv("MINTCCL_GEMM_BN")) {
-    const int v = atoi(e);
-    if (v == 224 || v == 256) return v;
-  }
   const long w256 = (long)((row_tiles * (N / 256) + nclusters - 1) / nclusters) * 256;
   const long w224 = (long)((row_tiles * (N / 224) + nclusters - 1) / nclusters) * 224;
   return w224 < w256 ? 224 : 256;
 }
+// The environment's tile width (MINTCCL_GEMM_BN), where the kernel has it; 0: none.
+static int forced_bn(int N, bool fp8, bool plain, bool tb) {
+  const char* e = getenv("MINTCCL_GEMM_BN");
+  const int v = e ? atoi(e) : 0;
+  if (v == 256 || (v == 224 && !fp8 && N % 224 == 0) || (plain && v == 128) || (plain && v == 64 && !fp8 && !tb)) return v;
+  return 0;
+}
+static int pick_bn(int row_tiles, int N, int nclusters, bool fp8) {
+  const int f = forced_bn(N, fp8, false, false);
+  return f ? f : pick_wide(row_tiles, N, nclusters, fp8);
+}
+// The same for a plain GEMM, where narrow tiles are to be had too.  The time of a wave in tenths of a 256-column k-block
+// (580 cycles): 9 a k-block for 224 columns, 5.5 for 128 (290 - 320 cycles), 4 for 64 (220: A's bytes do not shrink with
+// the tile), and one k-block to drain the last accumulator.  So a problem with too few wide tiles for the chip takes
+// the widest ones that fill it.  Measured (us, 256 / 128 / 64 columns): 128 x 4096 x 1792 13.7 / 9.1 / 7.9,
+// 512 x 4096 x 1792 14.5 / 9.9 / 12.1, 1024 x 1792 x 4096 24.8 / 15.6 / 20.5, 2048 x 4096 x 2048 26.3 / 25.3 / 33.0.
+static int pick_plain_bn(int row_tiles, int N, int kblocks, int nclusters, bool fp8, bool tb) {
+  if (const int f = forced_bn(N, fp8, true, tb)) return f;
+  const int wide = pick_wide(row_tiles, N, nclusters, fp8);
+  if (nclusters < 1) return wide;
+  auto cost = [&](int bn, int per2) {   // twice the tenths
+    return (long)((row_tiles * (N / bn) + nclusters - 1) / nclusters) * (kblocks * per2 + 20);
+  };
+  int best = wide;
+  long c = cost(wide, wide == 224 ? 18 : 20);
+  if (cost(128, 11) < c) {
+    best = 128;
+    c = cost(128, 11);
+  }
+  if (!fp8 && !tb && cost(64, 8) < c) best = 64;
+  return best;
+}
 
 static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N,
                      int K, int ldc, int nctas, bool fp8, bool ta = false, bool tb = false, int epi = mt::EPI_NONE,
-                     void* aux = nullptr) {
+                     void* aux = nullptr, int stat = -1) {
   int dev = 0;
   cudaGetDevice(&dev);
   const int row_tiles = (M + 255) / 256;
@@ -146,7 +173,7 @@ static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B
     const int fit = mt::gemm_pair_max_clusters(mt::MODE_PLAIN, fp8);
     if (fit > 0 && ncl > fit) ncl = fit;
   }
-  const int bn = pick_bn(row_tiles, N, ncl, fp8);
+  const int bn = pick_plain_bn(row_tiles, N, K / (fp8 ? 128 : 64), ncl, fp8, tb);
   mt::GemmMaps maps;
   mt::PairSfMaps sf;
   memset(&maps, 0, sizeof(maps));
@@ -179,7 +206,7 @@ static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B
   if (nclusters < 1) nclusters = 1;
   cudaError_t e = mt::launch_gemm_pair(mt::MODE_PLAIN, maps, sf, a, nclusters, 1, (cudaStream_t)stream, fp8, bn);
   if (e != cudaSuccess) return fail(std::string("pair gemm launch: ") + cudaGetErrorString(e));
-  mthost::stat_add(fp8 ? mthost::ST_GEMM_MXFP8 : mthost::ST_GEMM, (uint64_t)(2.0 * M * N * K));
+  mthost::stat_add(stat >= 0 ? stat : (fp8 ? mthost::ST_GEMM_MXFP8 : mthost::ST_GEMM), (uint64_t)(2.0 * M * N * K));
   return 0;
 }
 
@@ -194,7 +221,7 @@ void mt_gemm_set_pair(int mode) { g_pair_mode = mode; }
 int mt_gemm(void* stream, const void* A, const void* B, void* C, int M, int N, int K, int ldc, int nctas) {
   if (check_shape(M, N, K, 1)) return -1;
   if (ldc < N || ldc % 8 || ((uintptr_t)C & 15)) return fail("C must be 16-byte aligned with ldc >= N, ldc % 8 == 0");
-  if (use_pair(M)) return gemm_pair(stream, A, nullptr, B, nullptr, C, M, N, K, ldc, nctas, false);
+  if (pair_on()) return gemm_pair(stream, A, nullptr, B, nullptr, C, M, N, K, ldc, nctas, false);
   int dev = 0;
   cudaGetDevice(&dev);
   mt::GemmMaps maps;
@@ -245,7 +272,7 @@ int mt_gemm_mxfp8(void* stream, const void* A, const void* sfa, const void* B, c
   if (check_shape(M, N, K, 1) || K % 128) return fail("MXFP8 GEMM: M multiple of 128, N of 256, K of 128");
   if (ldc < N || ldc % 8 || ((uintptr_t)C & 15)) return fail("C must be 16-byte aligned with ldc >= N, ldc % 8 == 0");
   if (((uintptr_t)sfa | (uintptr_t)sfb) & 15) return fail("scale tensors must be 16-byte aligned");
-  if (use_pair(M)) return gemm_pair(stream, A, sfa, B, sfb, C, M, N, K, ldc, nctas, true);
+  if (pair_on()) return gemm_pair(stream, A, sfa, B, sfb, C, M, N, K, ldc, nctas, true);
   int dev = 0;
   cudaGetDevice(&dev);
   mt::GemmMaps maps;
@@ -311,9 +338,12 @@ static int ag_gemm_impl(MtComm* c, void* stream, const void* const* a_shard, con
       a.aux[lr] = act[lr];
     }
     a.epi = mt::EPI_SILU;
-    if (n == 1)   // nothing to gather (M % 256 == 128 included)
-      return gemm_pair(stream, a_shard[0], nullptr, B[0], nullptr, C[0], M, N, K, ldc, nctas, false, false, false, mt::EPI_SILU, act[0]);
-    if (!use_pair(M / n) || comm_mode == 2) return fail("the fused activation runs on CTA pairs");
+    if (n > 1 && (!use_pair(M / n) || comm_mode == 2)) return fail("the fused activation runs on CTA pairs");
+  }
+  if (n == 1 && (pair_on() || act)) {   // nothing to gather: the product itself
+    if (((uintptr_t)C[0] & 15) || (fp8 && (((uintptr_t)sfa[0] | (uintptr_t)sfb[0]) & 15))) return fail("C and the scales must be 16-byte aligned");
+    return gemm_pair(stream, a_shard[0], fp8 ? sfa[0] : nullptr, B[0], fp8 ? sfb[0] : nullptr, C[0], M, N, K, ldc, nctas, fp8, false,
+                     false, a.epi, a.aux[0], mthost::ST_AG_GEMM);
   }
   if (n == 1) ncomm = 0;
   else if (ncomm < 1 || ncomm > 64) return fail("ncomm out of range");
@@ -410,10 +440,12 @@ static int gemm_rs_impl(MtComm* c, void* stream, const void* const* A, const voi
     // nothing to reduce: the product itself, without the staging area and the reducers' pass over it (8192 x 4096 x 1792:
     // 128 us with them, 83 without).  The sum of one bf16 partial tile is that tile, so the bytes are the same.
     if ((uintptr_t)out[0] & 15) return fail("out must be 16-byte aligned");
-    const int rc = tb ? gemm_pair(stream, A[0], nullptr, B[0], nullptr, out[0], M, N, K, N, nctas, false, false, true)
-                      : (fp8 ? mt_gemm_mxfp8(stream, A[0], sfa[0], B[0], sfb[0], out[0], M, N, K, N, nctas)
-                             : mt_gemm(stream, A[0], B[0], out[0], M, N, K, N, nctas));
-    return rc;
+    if (fp8 && (((uintptr_t)sfa[0] | (uintptr_t)sfb[0]) & 15)) return fail("scale tensors must be 16-byte aligned");
+    if (tb || pair_on())
+      return gemm_pair(stream, A[0], fp8 ? sfa[0] : nullptr, B[0], fp8 ? sfb[0] : nullptr, out[0], M, N, K, N, nctas, fp8, false, tb,
+                       mt::EPI_NONE, nullptr, mthost::ST_GEMM_RS);
+    return fp8 ? mt_gemm_mxfp8(stream, A[0], sfa[0], B[0], sfb[0], out[0], M, N, K, N, nctas)
+               : mt_gemm(stream, A[0], B[0], out[0], M, N, K, N, nctas);
   }
   if (tb && !use_pair(M / c->nranks)) return fail("a transposed B needs rows per rank that are a multiple of 256");
   int grid = nctas > 0 ? nctas : sm_count(c->device);

@@ -51,26 +51,38 @@ namespace pair {
 
 constexpr int BMC = 128;   // A rows (and accumulator rows) per CTA
 constexpr int BM2 = 256;   // rows of the pair's tile
-constexpr int BNC = 128;   // B rows staged by each CTA
-constexpr int STAGES = 6;
 constexpr int kThreads = 192;
-constexpr uint32_t A_BYTES = BMC * 128, B_BYTES = BNC * 128;  // rows of 128 bytes (64 bf16 or 128 fp8)
-constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr uint32_t A_BYTES = BMC * 128;   // rows of 128 bytes (64 bf16 or 128 fp8)
 constexpr int EPI_PITCH = 144;
 constexpr uint32_t EPI_BYTES = 4 * 32 * EPI_PITCH;
-constexpr uint32_t SF_STAGE_BYTES = 1536;  // MXFP8: scale atom of the CTA's A rows + two atoms for all 256 B rows
 constexpr uint32_t CTL_BYTES = 512;
-constexpr uint32_t SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + EPI_BYTES + CTL_BYTES + STAGES * SF_STAGE_BYTES;
 constexpr uint32_t TMEM_COLS = 512;
-static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
+constexpr uint32_t T_CHUNK = 64 * 128;    // 64 K rows of 64 columns of an operand stored transposed
+
+// Shared memory of one kernel form.  Narrow tiles move fewer bytes per k-block, so more stages keep as many in flight.
+template <int MODE, bool FP8, int TILE_N, bool TB>
+struct Shape {
+  static constexpr int BNC = TILE_N / 2;   // B rows staged by each CTA
+  static constexpr int STAGES = TILE_N >= 224 ? 6 : (TILE_N == 128 ? 8 : 10);
+  static constexpr uint32_t B_BYTES = BNC * 128;   // a multiple of 1024: whole 128-byte swizzle atoms
+  // transposed: whole 64-column chunks
+  static constexpr uint32_t B_PITCH = TB ? (uint32_t)((BNC + 63) / 64) * T_CHUNK : B_BYTES;
+  // MXFP8: scale atom of the CTA's A rows + those of all B rows of the tile
+  static constexpr uint32_t SF_STAGE_BYTES = FP8 ? 512 * (1 + TILE_N / 128) : 0;
+  static constexpr uint32_t RING = MODE == MODE_AG_GEMM ? fused::COMM_SLOTS * fused::COMM_PIECE : 0;   // comm CTAs reuse the stages
+  static constexpr uint32_t OPERANDS = STAGES * (A_BYTES + B_PITCH) > RING ? STAGES * (A_BYTES + B_PITCH) : RING;
+  static constexpr uint32_t EPI = MODE == MODE_PLAIN ? 0 : EPI_BYTES;   // transpose of GEMM -> reduce-scatter; comm CTAs
+  static constexpr uint32_t SMEM = 1024 + OPERANDS + EPI + CTL_BYTES + STAGES * SF_STAGE_BYTES;
+  static_assert(SMEM <= 232448, "shared memory of one CTA");
+};
+constexpr int MAX_STAGES = 10;
 
 struct Ctl {
-  uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], drain;
+  uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2], drain;
   uint32_t tmem_base;
   int abort;
 };
 static_assert(sizeof(Ctl) <= CTL_BYTES && sizeof(fused::CommCtl) <= CTL_BYTES, "control block");
-static_assert(STAGES * STAGE_BYTES >= fused::COMM_SLOTS * fused::COMM_PIECE, "the comm ring reuses the operand stages");
 static_assert(kThreads == fused::kGemmThreads, "comm and reducer code assumes this block size");
 
 __device__ int g_pair_error;  // set when a wait of this kernel expired (read by mt_gemm_pair_error)
@@ -125,6 +137,29 @@ __device__ __forceinline__ void load_row64(const uint8_t* p, uint32_t* v, bool w
   }
 }
 
+// The same for a whole warp: one answer for all lanes, so that the issue loops stay warp-uniform.
+__device__ __noinline__ bool wait_bar_warp_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint64_t timeout_ns) {
+  uint32_t spins = 0;
+  uint64_t t0 = 0;
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if ((++spins & 0x3ffu) == 0) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+      const uint64_t now = __shfl_sync(0xffffffffu, globaltimer(), 0);
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > timeout_ns) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint64_t timeout_ns) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return wait_bar_warp_slow(bar, parity, abort_flag, timeout_ns);
+}
+__device__ __forceinline__ bool aborted_warp(volatile int* abort_flag) { return __any_sync(0xffffffffu, *abort_flag != 0); }
+
 // silu and its derivative on two packed bf16, in fp32.  The exponential and the quotient are the fast forms (their
 // error is 1e-6, the result is rounded to 8 bits): with expf and an exact division the last tile's epilogue is longer
 // than what the torch pass costs.
@@ -165,31 +200,34 @@ __device__ __forceinline__ Tile tile_of(const GemmArgs& a, int lr, int t) {
   return mt_fused_tile(MODE, t, MODE == MODE_PLAIN ? (a.M + BM2 - 1) & ~(BM2 - 1) : a.M, a.N, a.nranks, a.rank[lr], a.raster, BM2, TILE_N);
 }
 
-// TILE_N: columns of a tile, 256 or 224.  224 exists for the wave count: 8192 x 1792 (the Llama-3-8B up projection on
-// 8 ranks) is 224 tiles of 256 x 256, 3.03 waves on 74 clusters, i.e. a fourth wave for two tiles; as 256 tiles of
-// 256 x 224 it is four waves of tiles that are an eighth smaller.  bf16 only (the MXFP8 scale atoms cover 128
-// rows of B) and not for GEMM -> reduce-scatter (its staging layout is in 256-column tiles).
+// TILE_N: columns of a tile.  256 moves the fewest operand bytes per product.  224 exists for the wave count: 8192 x 1792
+// (the Llama-3-8B up projection on 8 ranks) is 224 tiles of 256 x 256, 3.03 waves on 74 clusters, i.e. a fourth wave for
+// two tiles; as 256 tiles of 256 x 224 it is four waves of tiles that are an eighth smaller.  bf16 only (the MXFP8 scale
+// atoms cover 128 rows of B) and not for GEMM -> reduce-scatter (its staging layout is in 256-column tiles).  128 and 64
+// are for plain GEMMs that have too few 256-column tiles for the chip: a k-block of a narrow tile takes 0.55 / 0.4 of a
+// wide one's time and two or four times as many SMs work (host rule: pick_plain_bn).
 // TA, TB: the operand is stored transposed (compile-time: choosing descriptors in the issue loops cost 7 %).
 template <int MODE, bool FP8, int TILE_N, bool TA = false, bool TB = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ PairSfMaps sfmaps, GemmArgs a) {
-  static_assert(TILE_N == 256 || (TILE_N == 224 && !FP8 && MODE != MODE_GEMM_RS), "tile widths");
-  constexpr int BN = TILE_N, BNC = TILE_N / 2;             // shadow the 256-column constants of the namespace
-  constexpr uint32_t B_BYTES = BNC * 128;                   // a multiple of 1024: whole 128-byte swizzle atoms
-  constexpr uint32_t B_PITCH = 128 * 128;                   // a transposed B takes two whole 64-column chunks
-  constexpr uint32_t T_CHUNK = 64 * 128;                    // 64 K rows of 64 columns
+  static_assert(TILE_N == 256 || (TILE_N == 224 && !FP8 && MODE != MODE_GEMM_RS) || (TILE_N == 128 && MODE == MODE_PLAIN) ||
+                    (TILE_N == 64 && MODE == MODE_PLAIN && !FP8 && !TB), "tile widths");
+  using S = Shape<MODE, FP8, TILE_N, TB>;
+  constexpr int BN = TILE_N, BNC = S::BNC, STAGES = S::STAGES;
+  constexpr uint32_t B_BYTES = S::B_BYTES, B_PITCH = S::B_PITCH, SF_STAGE_BYTES = S::SF_STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   const int lr = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // through a shuffle: known to be the same in all lanes of the warp
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   // the same offsets in both CTAs: the MMA descriptors name shared memory of the pair by offset
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sA = smem;
   uint8_t* sB = smem + STAGES * A_BYTES;
-  uint8_t* sEpi = smem + STAGES * STAGE_BYTES;
-  Ctl* ctl = (Ctl*)(sEpi + EPI_BYTES);
-  uint8_t* sSF = sEpi + EPI_BYTES + CTL_BYTES;
+  uint8_t* sEpi = smem + S::OPERANDS;
+  Ctl* ctl = (Ctl*)(sEpi + S::EPI);
+  uint8_t* sSF = sEpi + S::EPI + CTL_BYTES;
   constexpr int BKE = FP8 ? 128 : 64;    // K elements per stage
-  constexpr uint32_t ACC = FP8 ? 1 : 2;  // accumulator buffers (MXFP8 keeps TMEM columns for the scales)
+  constexpr uint32_t ACC = FP8 && BN > 128 ? 1 : 2;  // accumulator buffers (MXFP8 keeps TMEM columns for the scales)
   const uint32_t cr = cluster_ctarank();
   const bool leader = cr == 0;
   const int nextra = MODE == MODE_PLAIN ? 0 : a.ncomm;  // AG: data movers, RS: dedicated reducers (whole clusters)
@@ -198,7 +236,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const uint64_t timeout_ns = a.timeout_ns;
 
   if (MODE == MODE_AG_GEMM && (int)blockIdx.x >= ngemm) {
-    fused::ag_comm_cta<FP8>(a, lr, (int)blockIdx.x - ngemm, nextra, smem, (fused::CommCtl*)(sEpi + EPI_BYTES));
+    fused::ag_comm_cta<FP8>(a, lr, (int)blockIdx.x - ngemm, nextra, smem, (fused::CommCtl*)(sEpi + S::EPI));
     return;
   }
   if (MODE == MODE_GEMM_RS && (int)blockIdx.x >= ngemm) {
@@ -229,7 +267,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers exist before anybody signals across
   tc_fence_after();
-  const uint32_t tmem_base = ctl->tmem_base;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
   volatile int* abort_flag = &ctl->abort;
 
   static_assert(!(TA || TB) || !FP8, "8-bit operands are K-major");
@@ -237,12 +275,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const int kblocks = a.K / BKE;
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer (one lane, both CTAs)
-    if (lane == 0) {
+    // ------------------------------------------------------------ TMA producer (both CTAs): a uniform warp, one lane issues
+    {
       const uint32_t empty_peer = map_to_cta(smem_u32(&ctl->empty[0]), 1), full_leader = map_to_cta(smem_u32(&ctl->full[0]), 0);
       uint32_t s = 0, ph = 0;   // stage and its parity: running counters, no division in the issue loops
       bool passed = false;      // the ring has been round once
-      for (int t = cluster_id; t < tiles && !*abort_flag; t += nclusters) {
+      for (int t = cluster_id; t < tiles && !aborted_warp(abort_flag); t += nclusters) {
         const Tile tc_ = tile_of<MODE, BN>(a, lr, t);
         int arow = tc_.mb * BM2 + (int)cr * BMC;
         const int brow = tc_.nb * BN + (int)cr * BNC;
@@ -259,7 +297,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             const uint64_t want = a.epoch * (uint64_t)a.comm_split;
             uint32_t spins = 0;
             uint64_t t0 = 0;
-            while (load64_acquire_sys(cnt) < want) {
+            while (load64_acquire_sys(cnt) < want) {   // every lane: each then orders its own loads behind the count
               if ((++spins & 0xffu) == 0) {
                 const uint64_t now = globaltimer();
                 if (t0 == 0) t0 = now;
@@ -270,34 +308,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 }
               }
             }
-            if (*abort_flag) break;
+            if (aborted_warp(abort_flag)) break;
             fence_proxy_async_global();  // peer stores (generic proxy) before our TMA reads (async proxy)
           }
         }
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (!wait_bar(&ctl->empty[s], ph ^ 1, abort_flag, timeout_ns)) break;
-          // the MMA thread's commit lands on the leader's barrier only: pass it on to the peer's producer
-          if (leader && passed) mbar_arrive_cluster(empty_peer + s * 8);
-          const uint32_t full0 = full_leader + s * 8;
-          if (leader) mbar_expect_tx(&ctl->full[s], 2 * (A_BYTES + (TB ? B_PITCH : B_BYTES) + (FP8 ? SF_STAGE_BYTES : 0)));
-          if (TA) {
-            tma_load_2d_pair(sA + s * A_BYTES, amap, arow, kb * BKE, full0);
-            tma_load_2d_pair(sA + s * A_BYTES + T_CHUNK, amap, arow + 64, kb * BKE, full0);
-          } else {
-            tma_load_2d_pair(sA + s * A_BYTES, amap, kb * BKE, arow, full0);
-          }
-          if (TB) {
-            tma_load_2d_pair(sB + s * B_PITCH, &maps.b[lr], brow, kb * BKE, full0);
-            tma_load_2d_pair(sB + s * B_PITCH + T_CHUNK, &maps.b[lr], brow + 64, kb * BKE, full0);
-          } else {
-            tma_load_2d_pair(sB + s * B_PITCH, &maps.b[lr], kb * BKE, brow, full0);
-          }
-          if (FP8) {
-            // scale atoms are rows of a [atoms, 128 x u32] tensor: atom (row block of 128, K block of 128)
-            uint8_t* sf = sSF + s * SF_STAGE_BYTES;
-            tma_load_2d_pair(sf, &sfmaps.sfa[lr], 0, sfa_row * kblocks + kb, full0);
-            tma_load_2d_pair(sf + 512, &sfmaps.sfb[lr], 0, (tc_.nb * 2) * kblocks + kb, full0);
-            tma_load_2d_pair(sf + 1024, &sfmaps.sfb[lr], 0, (tc_.nb * 2 + 1) * kblocks + kb, full0);
+          if (!wait_bar_warp(&ctl->empty[s], ph ^ 1, abort_flag, timeout_ns)) break;
+          if (elect_one()) {
+            // the MMA thread's commit lands on the leader's barrier only: pass it on to the peer's producer
+            if (leader && passed) mbar_arrive_cluster(empty_peer + s * 8);
+            const uint32_t full0 = full_leader + s * 8;
+            if (leader) mbar_expect_tx(&ctl->full[s], 2 * (A_BYTES + (TB ? B_PITCH : B_BYTES) + (FP8 ? SF_STAGE_BYTES : 0)));
+            if (TA) {
+              tma_load_2d_pair(sA + s * A_BYTES, amap, arow, kb * BKE, full0);
+              tma_load_2d_pair(sA + s * A_BYTES + T_CHUNK, amap, arow + 64, kb * BKE, full0);
+            } else {
+              tma_load_2d_pair(sA + s * A_BYTES, amap, kb * BKE, arow, full0);
+            }
+            if (TB) {
+              tma_load_2d_pair(sB + s * B_PITCH, &maps.b[lr], brow, kb * BKE, full0);
+              if (BNC > 64) tma_load_2d_pair(sB + s * B_PITCH + T_CHUNK, &maps.b[lr], brow + 64, kb * BKE, full0);
+            } else {
+              tma_load_2d_pair(sB + s * B_PITCH, &maps.b[lr], kb * BKE, brow, full0);
+            }
+            if (FP8) {
+              // scale atoms are rows of a [atoms, 128 x u32] tensor: atom (row block of 128, K block of 128)
+              uint8_t* sf = sSF + s * SF_STAGE_BYTES;
+              tma_load_2d_pair(sf, &sfmaps.sfa[lr], 0, sfa_row * kblocks + kb, full0);
+              tma_load_2d_pair(sf + 512, &sfmaps.sfb[lr], 0, (tc_.nb * (BN / 128)) * kblocks + kb, full0);
+              if (BN > 128) tma_load_2d_pair(sf + 1024, &sfmaps.sfb[lr], 0, (tc_.nb * 2 + 1) * kblocks + kb, full0);
+            }
           }
           if (++s == STAGES) {
             s = 0;
@@ -306,63 +346,68 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           }
         }
       }
-      if (*abort_flag) {
-        // copies this thread issued may still be landing in shared memory: give them a bounded time
+      if (aborted_warp(abort_flag)) {
+        // copies this warp issued may still be landing in shared memory: give them a bounded time
         const uint64_t t0 = globaltimer();
         while (globaltimer() - t0 < 100000ull) __nanosleep(1000);
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (one lane of the leader)
-    if (leader && lane == 0) {
+    // ------------------------------------------------------------ MMA issuer (leader): a uniform warp, one lane issues
+    // What bounds a k-block of any width is this loop: with a single-lane branch around it every operand went through a
+    // per-thread register, and wait, four MMAs and commit took 535 cycles (MXFP8, with its scale copies, 840) where the
+    // tensor cores need 512 for a 256-column tile and a quarter of that for a 64-column one.
+    if (leader) {
       constexpr uint32_t idesc = make_idesc_bf16(BM2, BN) | (TA ? kIdescTransA : 0u) | (TB ? kIdescTransB : 0u);
       constexpr uint32_t ka = TA ? 128 : 2, kb16 = TB ? 128 : 2;   // descriptor step of 16 elements along K
       const uint64_t da0 = TA ? make_smem_desc_mn_sw128(sA, T_CHUNK) : make_smem_desc_sw128(sA);
       const uint64_t db0 = TB ? make_smem_desc_mn_sw128(sB, T_CHUNK) : make_smem_desc_sw128(sB);
+      const uint64_t dsf0 = make_smem_desc_sf(sSF);
       const uint32_t empty0 = smem_u32(&ctl->empty[0]);
       uint32_t s = 0, ph = 0, tile_i = 0;
-      for (int t = cluster_id; t < tiles && !*abort_flag; t += nclusters, ++tile_i) {
+      for (int t = cluster_id; t < tiles && !aborted_warp(abort_flag); t += nclusters, ++tile_i) {
         const uint32_t as = tile_i % ACC, aph = (tile_i / ACC) & 1;
-        if (!wait_bar(&ctl->acc_empty[as], aph ^ 1, abort_flag, timeout_ns)) break;
+        if (!wait_bar_warp(&ctl->acc_empty[as], aph ^ 1, abort_flag, timeout_ns)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * BN;
         bool ok = true;
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (!wait_bar(&ctl->full[s], ph, abort_flag, timeout_ns)) {
+          if (!wait_bar_warp(&ctl->full[s], ph, abort_flag, timeout_ns)) {
             ok = false;
             break;
           }
           tc_fence_after();
           // descriptor addresses are in units of 16 bytes and stay below 2^14: no carry into the other fields
-          const uint64_t da = da0 + s * (A_BYTES >> 4), db = db0 + s * (B_PITCH >> 4);
-          if (FP8) {
-            const uint32_t tsfa = tmem_base + 256 + s * 16, tsfb = tsfa + 4;
-            const uint8_t* sf = sSF + s * SF_STAGE_BYTES;
-            tmem_cp_sf_pair(tsfa, make_smem_desc_sf(sf));
-            tmem_cp_sf_pair(tsfb, make_smem_desc_sf(sf + 512));
-            tmem_cp_sf_pair(tsfb + 4, make_smem_desc_sf(sf + 1024));
+          const uint64_t da = da0 + s * (A_BYTES >> 4), db = db0 + s * (B_PITCH >> 4), dsf = dsf0 + s * (SF_STAGE_BYTES >> 4);
+          const uint32_t tsfa = tmem_base + 256 + s * 16, tsfb = tsfa + 4, acc0 = kb > 0 ? 1u : 0u, bar = empty0 + s * 8;
+          if (elect_one()) {
+            if (FP8) {
+              tmem_cp_sf_pair(tsfa, dsf);
+              tmem_cp_sf_pair(tsfb, dsf + 32);
+              if (BN > 128) tmem_cp_sf_pair(tsfb + 4, dsf + 64);
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_mxfp8_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), make_idesc_mxfp8(BM2, BN, k, k), tsfa,
-                              tsfb, (kb > 0 || k > 0) ? 1u : 0u);
-          } else {
+              for (int k = 0; k < 4; ++k)
+                umma_mxfp8_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), make_idesc_mxfp8(BM2, BN, k, k), tsfa,
+                                tsfb, k > 0 ? 1u : acc0);
+            } else {
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              umma_bf16_pair(d_tmem, da + (uint64_t)(k * ka), db + (uint64_t)(k * kb16), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              for (int k = 0; k < 4; ++k)
+                umma_bf16_pair(d_tmem, da + (uint64_t)(k * ka), db + (uint64_t)(k * kb16), idesc, k > 0 ? 1u : acc0);
+            }
+            // the stage is free (in both CTAs) once these MMAs have read it
+            umma_commit_pair(bar);
           }
-          // the stage is free (in both CTAs) once these MMAs have read it
-          umma_commit_pair(empty0 + s * 8);
           if (++s == STAGES) {
             s = 0;
             ph ^= 1;
           }
         }
         if (!ok) break;
-        umma_commit_pair(smem_u32(&ctl->acc_full[as]));
+        if (elect_one()) umma_commit_pair(smem_u32(&ctl->acc_full[as]));
       }
       // no MMA may still be running when TMEM is freed, on the normal path or after an abort
-      umma_commit_pair(smem_u32(&ctl->drain));
-      wait_bar(&ctl->drain, 0, abort_flag, timeout_ns);
+      if (elect_one()) umma_commit_pair(smem_u32(&ctl->drain));
+      wait_bar_warp(&ctl->drain, 0, abort_flag, timeout_ns);
     }
   } else {
     // ------------------------------------------------------------ epilogue warps (2..5, both CTAs)
@@ -525,41 +570,62 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 }  // namespace pair
 
 // Operand forms of the bf16 kernels: 0 both K-major, 1 B stored transposed, 2 both stored transposed (plain GEMM only).
-static const void* pair_fn(int mode, bool fp8, int bn = 256, int form = 0) {
-  using pair::gemm_pair_kernel;
+struct PairKernel {
+  const void* fn;
+  uint32_t smem;
+};
+template <int MODE, bool FP8, int TILE_N, bool TA = false, bool TB = false>
+static PairKernel pair_kernel() {
+  return {(const void*)pair::gemm_pair_kernel<MODE, FP8, TILE_N, TA, TB>, pair::Shape<MODE, FP8, TILE_N, TB>::SMEM};
+}
+template <bool TA, bool TB>
+static PairKernel plain_kernel(int bn) {
+  switch (bn) {
+    case 256: return pair_kernel<MODE_PLAIN, false, 256, TA, TB>();
+    case 224: return pair_kernel<MODE_PLAIN, false, 224, TA, TB>();
+    case 128: return pair_kernel<MODE_PLAIN, false, 128, TA, TB>();
+    default: return {nullptr, 0};
+  }
+}
+static PairKernel pair_fn(int mode, bool fp8, int bn = 256, int form = 0) {
+  const PairKernel none = {nullptr, 0};
   if (fp8) {
-    if (bn != 256 || form) return nullptr;
+    if (form) return none;
+    if (bn == 128) return mode == MODE_PLAIN ? pair_kernel<MODE_PLAIN, true, 128>() : none;
+    if (bn != 256) return none;
     switch (mode) {
-      case MODE_PLAIN: return (const void*)gemm_pair_kernel<MODE_PLAIN, true, 256>;
-      case MODE_AG_GEMM: return (const void*)gemm_pair_kernel<MODE_AG_GEMM, true, 256>;
-      case MODE_GEMM_RS: return (const void*)gemm_pair_kernel<MODE_GEMM_RS, true, 256>;
-      default: return nullptr;
+      case MODE_PLAIN: return pair_kernel<MODE_PLAIN, true, 256>();
+      case MODE_AG_GEMM: return pair_kernel<MODE_AG_GEMM, true, 256>();
+      case MODE_GEMM_RS: return pair_kernel<MODE_GEMM_RS, true, 256>();
+      default: return none;
     }
   }
   if (mode == MODE_PLAIN) {
-    if (form == 1) return bn == 224 ? (const void*)gemm_pair_kernel<MODE_PLAIN, false, 224, false, true>
-                                    : (const void*)gemm_pair_kernel<MODE_PLAIN, false, 256, false, true>;
-    if (form == 2) return bn == 224 ? (const void*)gemm_pair_kernel<MODE_PLAIN, false, 224, true, true>
-                                    : (const void*)gemm_pair_kernel<MODE_PLAIN, false, 256, true, true>;
-    return bn == 224 ? (const void*)gemm_pair_kernel<MODE_PLAIN, false, 224> : (const void*)gemm_pair_kernel<MODE_PLAIN, false, 256>;
+    if (form == 1) return plain_kernel<false, true>(bn);
+    if (form == 2) return plain_kernel<true, true>(bn);
+    return bn == 64 ? pair_kernel<MODE_PLAIN, false, 64>() : plain_kernel<false, false>(bn);
   }
-  if (mode == MODE_AG_GEMM && form == 0)
-    return bn == 224 ? (const void*)gemm_pair_kernel<MODE_AG_GEMM, false, 224> : (const void*)gemm_pair_kernel<MODE_AG_GEMM, false, 256>;
-  if (mode == MODE_GEMM_RS && bn == 256)
-    return form == 1 ? (const void*)gemm_pair_kernel<MODE_GEMM_RS, false, 256, false, true>
-                     : (form == 0 ? (const void*)gemm_pair_kernel<MODE_GEMM_RS, false, 256> : nullptr);
-  return nullptr;
+  if (mode == MODE_AG_GEMM && form == 0) {
+    if (bn == 224) return pair_kernel<MODE_AG_GEMM, false, 224>();
+    return bn == 256 ? pair_kernel<MODE_AG_GEMM, false, 256>() : none;
+  }
+  if (mode == MODE_GEMM_RS && bn == 256) {
+    if (form == 1) return pair_kernel<MODE_GEMM_RS, false, 256, false, true>();
+    return form == 0 ? pair_kernel<MODE_GEMM_RS, false, 256>() : none;
+  }
+  return none;
 }
 
 // Clusters of this kernel that the device can hold at once.  The kernel is persistent (cluster i takes tiles
 // i, i + n, ...), so a grid with more clusters than fit would run its tail after the rest has finished.
 int gemm_pair_max_clusters(int mode, bool fp8, int bn, int form) {
-  static int cached[36] = {};
-  const void* fn = pair_fn(mode, fp8, bn, form);
-  if (!fn) return 0;
-  int& slot = cached[((mode * 2 + (fp8 ? 1 : 0)) * 2 + (bn == 224 ? 1 : 0)) * 3 + form];
+  static int cached[72] = {};
+  const PairKernel k = pair_fn(mode, fp8, bn, form);
+  if (!k.fn) return 0;
+  const int width = bn == 256 ? 0 : (bn == 224 ? 1 : (bn == 128 ? 2 : 3));
+  int& slot = cached[((mode * 2 + (fp8 ? 1 : 0)) * 4 + width) * 3 + form];
   if (slot > 0) return slot;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::SMEM_BYTES) != cudaSuccess) return 0;
+  if (cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem) != cudaSuccess) return 0;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -567,7 +633,7 @@ int gemm_pair_max_clusters(int mode, bool fp8, int bn, int form) {
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(sms & ~1);
   cfg.blockDim = dim3(pair::kThreads);
-  cfg.dynamicSmemBytes = pair::SMEM_BYTES;
+  cfg.dynamicSmemBytes = k.smem;
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeClusterDimension;
   at.val.clusterDim.x = 2;
@@ -576,7 +642,7 @@ int gemm_pair_max_clusters(int mode, bool fp8, int bn, int form) {
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess || n <= 0) {
+  if (cudaOccupancyMaxActiveClusters(&n, k.fn, &cfg) != cudaSuccess || n <= 0) {
     cudaGetLastError();
     n = sms / 2;
   }
@@ -592,8 +658,8 @@ int gemm_pair_max_clusters(int mode, bool fp8, int bn, int form) {
 cudaError_t launch_gemm_pair(int mode, const GemmMaps& maps, const PairSfMaps& sf, const GemmArgs& a, int nclusters,
                              int nlocal, cudaStream_t s, bool fp8, int bn) {
   const int form = a.ta ? 2 : (a.tb ? 1 : 0);
-  const void* fn = pair_fn(mode, fp8, bn, form);
-  if (!fn || (a.ta && !a.tb)) return cudaErrorInvalidValue;
+  const PairKernel k = pair_fn(mode, fp8, bn, form);
+  if (!k.fn || (a.ta && !a.tb)) return cudaErrorInvalidValue;
   const int fit = gemm_pair_max_clusters(mode, fp8, bn, form);  // also sets the shared-memory attribute once
   if (fit <= 0) return cudaErrorInvalidValue;
   const int extra = mode == MODE_PLAIN ? 0 : a.ncomm;
@@ -609,20 +675,20 @@ cudaError_t launch_gemm_pair(int mode, const GemmMaps& maps, const PairSfMaps& s
   void* p[] = {(void*)&m, (void*)&sm, (void*)&args};
   count_launch();
   const dim3 grid(2 * nclusters + extra, nlocal);
-  if (nlocal == 1) return cudaLaunchKernel(fn, grid, dim3(pair::kThreads), p, pair::SMEM_BYTES, s);
+  if (nlocal == 1) return cudaLaunchKernel(k.fn, grid, dim3(pair::kThreads), p, k.smem, s);
   // emulated ranks wait on each other inside one grid: every CTA has to be resident
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = grid;
   cfg.blockDim = dim3(pair::kThreads);
-  cfg.dynamicSmemBytes = pair::SMEM_BYTES;
+  cfg.dynamicSmemBytes = k.smem;
   cfg.stream = s;
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeCooperative;
   at.val.cooperative = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelExC(&cfg, fn, p);
+  return cudaLaunchKernelExC(&cfg, k.fn, p);
 }
 
 int gemm_pair_error() {

@@ -131,7 +131,7 @@ int mt_ag_gemm_silu(MtComm* c, void* stream, const void* const* a_shard, const v
                     int nctas, int comm_mode, uint64_t shard_off, int comm_split);
 int mt_gemm_rs_t(MtComm* c, void* stream, const void* const* A, const void* const* B, void* const* out,
                  uint64_t stage_off, uint64_t flags_off, uint64_t epoch, int M, int N, int K, int nred, int nctas);
-// Plain GEMMs with M % 256 == 0 run on CTA pairs (tcgen05 cta_group::2) when MINTCCL_GEMM_PAIR is not 0; a wait
+// Plain GEMMs run on CTA pairs (tcgen05 cta_group::2) when MINTCCL_GEMM_PAIR is not 0; a wait
 // of that kernel that expired leaves 1 here (synchronises the device).
 int mt_gemm_pair_error(void);
 void mt_gemm_set_pair(int mode);                          // 1 pairs, 0 single CTA, -1 environment / default

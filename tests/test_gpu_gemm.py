@@ -247,3 +247,32 @@ def test_silu_derivative_in_the_epilogue(shape):
     want = da * (sig * (1 + h.float() * (1 - sig)))
     # one rounding; where 1 + h (1 - sig) cancels the fp32 factor itself is 1e-6 off
     assert bool(((got.float() - want).abs() <= 2 ** -8 * 1.001 * want.abs() + 4e-6 * da.abs()).all())
+
+
+@pytest.mark.parametrize("form", ["plain", "tb", "ta_tb", "dsilu", "mxfp8"])
+@pytest.mark.parametrize("bn", ["128", "64"])
+@pytest.mark.parametrize("shape", [(128, 256, 128), (256, 512, 1152), (640, 1792, 512), (2432, 768, 256)])
+def test_narrow_tiles_give_the_bits_of_wide_ones(shape, bn, form, monkeypatch):
+    """The tiles of problems with too few 256-column ones (forced here; 64 columns exist for K-major bf16 only and fall
+    back): every output is summed over K in the same order, so the bits are those of 256-column tiles."""
+    from mintccl_b200.ops import gemm as G
+    from mintccl_b200.ops import mxfp8 as mx
+    M, Nn, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + Nn + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(Nn, K, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    h = torch.randn(M, Nn, generator=g, device="cuda").to(torch.bfloat16)
+    at, wt = a.t().contiguous(), w.t().contiguous()
+    qa, qw = mx.quantize_rows_mxfp8(a), mx.quantize_rows_mxfp8(w)
+    call = {"plain": lambda: G.gemm(a, w), "tb": lambda: G.gemm_t(a, wt, tb=True), "ta_tb": lambda: G.gemm_t(at, wt, True, True),
+            "dsilu": lambda: G.gemm_dsilu(a, wt, h), "mxfp8": lambda: mx.gemm_mxfp8(*qa, *qw)}[form]
+    monkeypatch.setenv("MINTCCL_GEMM_BN", bn)
+    out = call()
+    monkeypatch.setenv("MINTCCL_GEMM_BN", "256")
+    wide = call()
+    monkeypatch.delenv("MINTCCL_GEMM_BN")
+    chosen = call()
+    torch.cuda.synchronize()
+    if form == "plain":
+        close(out, ref_mm(a, w), K)
+    assert torch.equal(out, wide) and torch.equal(chosen, wide)
