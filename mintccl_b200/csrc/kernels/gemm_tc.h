@@ -17,11 +17,13 @@ enum GemmEpi : int {
 };
 
 // TMA descriptors, one set per local rank (index 0 outside single-GPU emulation).
-struct GemmMaps {
-  CUtensorMap a[MT_MAX_RANKS];   // A operand: [M, K] (AG_GEMM: the gathered buffer)
-  CUtensorMap b[MT_MAX_RANKS];   // B operand: [N, K]
-  CUtensorMap a2[MT_MAX_RANKS];  // AG_GEMM: this rank's own rows [M / n, K]
+template <int NR>
+struct GemmMapsN {
+  CUtensorMap a[NR];   // A operand: [M, K] (AG_GEMM: the gathered buffer)
+  CUtensorMap b[NR];   // B operand: [N, K]
+  CUtensorMap a2[NR];  // AG_GEMM: this rank's own rows [M / n, K]
 };
+typedef GemmMapsN<MT_MAX_RANKS> GemmMaps;
 
 struct GemmArgs {
   void* c[MT_MAX_RANKS];               // output: C [M, ldc] (GEMM_RS: this rank's rows [M / n, N])
@@ -57,10 +59,12 @@ cudaError_t launch_gemm_tc(int mode, const GemmMaps& maps, const GemmArgs& a, in
 
 // ---- GEMM on CTA pairs (gemm_tc2.cu): one 256 x 256 tile per cluster of two CTAs, same modes and arguments ----
 // GemmMaps for this kernel: boxes of 128 rows x 128 bytes for A and for B (each CTA of a pair loads half of B).
-struct PairSfMaps {
-  CUtensorMap sfa[MT_MAX_RANKS];  // MXFP8: tiled scales of (the gathered) A as [atoms, 128] u32, box = one 512-byte atom
-  CUtensorMap sfb[MT_MAX_RANKS];  // same for B
+template <int NR>
+struct PairSfMapsN {
+  CUtensorMap sfa[NR];  // MXFP8: tiled scales of (the gathered) A as [atoms, 128] u32, box = one 512-byte atom
+  CUtensorMap sfb[NR];  // same for B
 };
+typedef PairSfMapsN<MT_MAX_RANKS> PairSfMaps;
 // bn: columns of a tile: 256, 224 (bf16, plain GEMM and all-gather -> GEMM), 128 (plain GEMM), 64 (bf16 plain GEMM, B
 // K-major); the map of B has boxes of bn / 2 rows
 cudaError_t launch_gemm_pair(int mode, const GemmMaps& maps, const PairSfMaps& sf, const GemmArgs& a, int nclusters,

@@ -206,10 +206,15 @@ __device__ __forceinline__ Tile tile_of(const GemmArgs& a, int lr, int t) {
 // atoms cover 128 rows of B) and not for GEMM -> reduce-scatter (its staging layout is in 256-column tiles).  128 and 64
 // are for plain GEMMs that have too few 256-column tiles for the chip: a k-block of a narrow tile takes 0.55 / 0.4 of a
 // wide one's time and two or four times as many SMs work (host rule: pick_plain_bn).
+// A plain GEMM has one set of descriptors: 0.6 KB of kernel parameters instead of 5 (1 us of a launch).
+template <int MODE>
+constexpr int kMaps = MODE == MODE_PLAIN ? 1 : MT_MAX_RANKS;
+
 // TA, TB: the operand is stored transposed (compile-time: choosing descriptors in the issue loops cost 7 %).
 template <int MODE, bool FP8, int TILE_N, bool TA = false, bool TB = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-    gemm_pair_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ PairSfMaps sfmaps, GemmArgs a) {
+    gemm_pair_kernel(const __grid_constant__ GemmMapsN<kMaps<MODE>> maps, const __grid_constant__ PairSfMapsN<kMaps<MODE>> sfmaps,
+                     GemmArgs a) {
   static_assert(TILE_N == 256 || (TILE_N == 224 && !FP8 && MODE != MODE_GEMM_RS) || (TILE_N == 128 && MODE == MODE_PLAIN) ||
                     (TILE_N == 64 && MODE == MODE_PLAIN && !FP8 && !TB), "tile widths");
   using S = Shape<MODE, FP8, TILE_N, TB>;
@@ -666,13 +671,25 @@ cudaError_t launch_gemm_pair(int mode, const GemmMaps& maps, const PairSfMaps& s
   if (extra & 1) return cudaErrorInvalidValue;
   if ((nclusters + extra / 2) * nlocal > fit) nclusters = fit / nlocal - extra / 2;
   if (nclusters < 1) return cudaErrorInvalidValue;
-  GemmMaps m = maps;
-  PairSfMaps sm = sf;
+  GemmMaps m;
+  PairSfMaps sm;
+  GemmMapsN<1> m1;
+  PairSfMapsN<1> sm1;
+  if (mode == MODE_PLAIN) {
+    m1.a[0] = maps.a[0];
+    m1.b[0] = maps.b[0];
+    m1.a2[0] = maps.a2[0];
+    sm1.sfa[0] = sf.sfa[0];
+    sm1.sfb[0] = sf.sfb[0];
+  } else {
+    m = maps;
+    sm = sf;
+  }
   GemmArgs args = a;
   uint64_t mis = (uint64_t)a.ldc * 2;
   for (int lr = 0; lr < nlocal; ++lr) mis |= (uint64_t)(uintptr_t)a.c[lr] | (uint64_t)(uintptr_t)a.aux[lr];
   args.wide_out = (mis & 31) == 0;
-  void* p[] = {(void*)&m, (void*)&sm, (void*)&args};
+  void* p[] = {mode == MODE_PLAIN ? (void*)&m1 : (void*)&m, mode == MODE_PLAIN ? (void*)&sm1 : (void*)&sm, (void*)&args};
   count_launch();
   const dim3 grid(2 * nclusters + extra, nlocal);
   if (nlocal == 1) return cudaLaunchKernel(k.fn, grid, dim3(pair::kThreads), p, k.smem, s);

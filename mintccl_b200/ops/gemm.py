@@ -39,7 +39,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, n
     if out is None:
         out = torch.empty(M, Nn, device=a.device, dtype=torch.bfloat16)
     _check(out, "out")
-    stream = torch.cuda.current_stream(a.device).cuda_stream
+    stream = N.raw_stream(a.get_device())
     if N.lib().mt_gemm(stream, a.data_ptr(), w.data_ptr(), out.data_ptr(), M, Nn, K, out.stride(0), nctas) < 0:
         raise RuntimeError(f"mt_gemm: {N.last_error()}")
     return out
@@ -58,7 +58,7 @@ def gemm_t(a: torch.Tensor, b: torch.Tensor, ta: bool = False, tb: bool = False)
     if K != K2:
         raise ValueError("inner dimensions differ")
     out = torch.empty(M, Nn, device=a.device, dtype=torch.bfloat16)
-    stream = torch.cuda.current_stream(a.device).cuda_stream
+    stream = N.raw_stream(a.get_device())
     if N.lib().mt_gemm_t(stream, a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, int(ta), int(tb)) < 0:
         raise RuntimeError(f"mt_gemm_t: {N.last_error()}")
     return out
@@ -71,7 +71,7 @@ def gemm_dsilu(d: torch.Tensor, w: torch.Tensor, h: torch.Tensor) -> torch.Tenso
     if d.shape[1] != w.shape[0] or tuple(h.shape) != (d.shape[0], w.shape[1]):
         raise ValueError("operand shapes do not match")
     out = torch.empty_like(h)
-    stream = torch.cuda.current_stream(d.device).cuda_stream
+    stream = N.raw_stream(d.get_device())
     if N.lib().mt_gemm_dsilu(stream, d.data_ptr(), w.data_ptr(), h.data_ptr(), out.data_ptr(), d.shape[0], w.shape[1], d.shape[1]) < 0:
         raise RuntimeError(f"mt_gemm_dsilu: {N.last_error()}")
     return out

@@ -41,17 +41,26 @@ def _plain_cuda(t: torch.Tensor) -> bool:
 
 
 def _native_quantize(flat: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
-    """One kernel (``csrc/kernels/mxfp8_quant.cu``) for contiguous ``[blocks, 32]`` on the GPU."""
+    """One kernel (``csrc/kernels/mxfp8_quant.cu``) for a contiguous tensor of whole blocks on the GPU."""
     if flat.data_ptr() % 16:
-        flat = flat.clone()      # a slice that starts off a 16-byte boundary
+        flat = flat.detach().clone()      # a slice that starts off a 16-byte boundary
     n = flat.numel()
     data = torch.empty(n, device=flat.device, dtype=torch.uint8)
     scale = torch.empty(n // BLOCK, device=flat.device, dtype=torch.uint8)
-    with torch.cuda.device(flat.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        if N.lib().mt_mxfp8_quantize(stream, _QUANT_DT[flat.dtype], flat.data_ptr(), data.data_ptr(), scale.data_ptr(), n) < 0:
-            raise RuntimeError(f"mt_mxfp8_quantize: {N.last_error()}")
+    _on_device(flat, N.lib().mt_mxfp8_quantize, _QUANT_DT[flat.dtype], flat.data_ptr(), data.data_ptr(), scale.data_ptr(), n)
     return data, scale
+
+
+def _on_device(t: torch.Tensor, fn, *args) -> None:
+    """``fn(current stream of t's device, *args)`` with that device current."""
+    dev = t.get_device()
+    if dev == torch.cuda.current_device():
+        rc = fn(N.raw_stream(dev), *args)
+    else:
+        with torch.cuda.device(dev):
+            rc = fn(N.raw_stream(dev), *args)
+    if rc < 0:
+        raise RuntimeError(f"{fn.__name__}: {N.last_error()}")
 
 
 _QUANT_DT = {torch.float32: N.DT_F32, torch.float16: N.DT_F16, torch.bfloat16: N.DT_BF16}
@@ -60,7 +69,9 @@ _QUANT_DT = {torch.float32: N.DT_F32, torch.float16: N.DT_F16, torch.bfloat16: N
 def quantize_mxfp8(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """fp32/bf16/fp16 tensor (numel a multiple of 32) -> (payload uint8 [numel], scales uint8 [numel / 32])."""
     if x.dtype in _QUANT_DT and _plain_cuda(x):
-        return _native_quantize(x.detach().reshape(-1, BLOCK).contiguous())
+        if x.numel() % BLOCK == 0 and x.is_contiguous():
+            return _native_quantize(x)
+        return _native_quantize(x.detach().reshape(-1, BLOCK).contiguous())    # refuses a ragged last block
     return _torch_quantize(x)
 
 
@@ -156,9 +167,7 @@ def tile_scales(scale: torch.Tensor) -> torch.Tensor:
     if (scale.dtype is torch.uint8 and scale.is_contiguous() and scale.numel() and scale.data_ptr() % 4 == 0
             and rows < 128 << 16 and _plain_cuda(scale)):
         out = torch.empty(rows * kb, device=scale.device, dtype=torch.uint8)
-        with torch.cuda.device(scale.device):
-            if N.lib().mt_mxfp8_tile_scales(torch.cuda.current_stream().cuda_stream, scale.data_ptr(), out.data_ptr(), rows, kb) < 0:
-                raise RuntimeError(f"mt_mxfp8_tile_scales: {N.last_error()}")
+        _on_device(scale, N.lib().mt_mxfp8_tile_scales, scale.data_ptr(), out.data_ptr(), rows, kb)
         return out
     return _torch_tile_scales(scale)
 
@@ -179,7 +188,7 @@ def gemm_mxfp8(a_data: torch.Tensor, a_scale: torch.Tensor, w_data: torch.Tensor
     if out is None:
         out = torch.empty(M, Nn, device=a_data.device, dtype=torch.bfloat16)
     sfa, sfb = (a_scale, w_scale) if scales_tiled else (tile_scales(a_scale), tile_scales(w_scale))
-    stream = torch.cuda.current_stream(a_data.device).cuda_stream
+    stream = N.raw_stream(a_data.get_device())
     rc = N.lib().mt_gemm_mxfp8(stream, a_data.data_ptr(), sfa.data_ptr(), w_data.data_ptr(), sfb.data_ptr(),
                                out.data_ptr(), M, Nn, K, out.stride(0), nctas)
     if rc < 0:

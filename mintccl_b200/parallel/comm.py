@@ -420,13 +420,16 @@ class Communicator:
         return ts
 
     def _stream(self) -> int:
-        return torch.cuda.current_stream(self.device).cuda_stream
+        return N.raw_stream(self.device)
 
     def _symm_off_all(self, ts: List[torch.Tensor]) -> Optional[int]:
-        offs = [self.symm_offset(t, lr) for lr, t in enumerate(ts)]
-        if offs[0] is None or any(o != offs[0] for o in offs):
+        off = ts[0].data_ptr() - self.heap_base[0]
+        if off < self.user_off:
             return None
-        return offs[0]
+        for base, t in zip(self.heap_base, ts):
+            if t.data_ptr() - base != off or off + t.nbytes > self.heap_bytes:
+                return None
+        return off
 
     def _ring_channels(self, nbytes: int, proto: int, nch: Optional[int]) -> int:
         cap = self.cfg.num_blocks or self.cfg.max_channels
@@ -660,7 +663,7 @@ class Communicator:
     # on: both buffers (address, size, type), the per-call arguments, and the process-wide settings that may
     # change between calls (``cfg.algo``, ``cfg.proto``, the route mode).
     def _run(self, fn, args) -> None:
-        if fn(self._handle, torch.cuda.current_stream(self.device).cuda_stream, *args) < 0:
+        if fn(self._handle, N.raw_stream(self.device), *args) < 0:
             raise RuntimeError(f"{fn.__name__}: {N.last_error()}")
         if self._rec_key is not None:
             if len(self._plans) > 8192:
@@ -673,7 +676,7 @@ class Communicator:
         if p is None:
             self._rec_key = key
             return False
-        if p[0](self._handle, torch.cuda.current_stream(self.device).cuda_stream, *p[1]) < 0:
+        if p[0](self._handle, N.raw_stream(self.device), *p[1]) < 0:
             raise RuntimeError(f"{p[0].__name__}: {N.last_error()}")
         return True
 
@@ -683,7 +686,7 @@ class Communicator:
 
     @staticmethod
     def _nbytes(t: torch.Tensor) -> int:
-        return t.numel() * t.element_size()
+        return t.nbytes
 
     def _check_out(self, what: str, ins, outs, in_numel: int, allow_cast: bool = True) -> None:
         """``out`` must hold exactly the result: the element count is fixed by the input, the element type is the
