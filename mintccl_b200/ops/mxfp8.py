@@ -32,12 +32,19 @@ def scale_to_float(scale: torch.Tensor) -> torch.Tensor:
     return torch.pow(2.0, scale.float() - 127.0)
 
 
+def _is_plain(t: torch.Tensor) -> bool:
+    """Whether ``t`` stands for its own memory: not a subclass, nothing that transforms it (vmap, functionalisation, a lazy
+    zero or negation), and nobody recording or replacing the operations on it (tracing, compilation, a dispatch mode).  All
+    of those go through the torch expressions below: a kernel launched from here would be missing from a recorded graph."""
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and t.layout is torch.strided
+            and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling()
+            and not torch._C._functorch.is_functorch_wrapped_tensor(t) and not torch._is_functional_tensor(t)
+            and not t.is_neg() and not t._is_zerotensor() and torch._C._len_torch_dispatch_stack() == 0)
+
+
 def _plain_cuda(t: torch.Tensor) -> bool:
-    """A tensor whose memory a kernel may be pointed at: not a subclass, not traced, vmapped or under a dispatch mode
-    (those go through the torch expressions below)."""
-    return (type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.layout is torch.strided
-            and not torch.compiler.is_compiling() and not torch._C._functorch.is_functorch_wrapped_tensor(t)
-            and not t.is_neg() and torch._C._len_torch_dispatch_stack() == 0)
+    """A tensor whose memory a kernel may be pointed at."""
+    return t.is_cuda and _is_plain(t)
 
 
 def _native_quantize(flat: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:

@@ -83,3 +83,70 @@ def test_sum_of_quantised_tensors_requantises_once():
     exact = sum(xs)
     rel = ((out - exact).norm() / exact.norm()).item()
     assert rel < 0.05
+
+
+class _Sub(torch.Tensor):
+    pass
+
+
+class _Mode(torch.utils._python_dispatch.TorchDispatchMode):
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.fixture
+def no_kernels(monkeypatch):
+    """The device condition lifted, and a kernel launch an error: what reaches it on the GPU would read raw memory."""
+    def launch(*a):
+        raise AssertionError("a kernel was launched on a tensor that is not its own memory")
+    monkeypatch.setattr(mx, "_plain_cuda", mx._is_plain)
+    monkeypatch.setattr(mx, "_on_device", launch)
+    with pytest.raises(AssertionError):
+        mx.quantize_mxfp8(torch.randn(64))                           # the condition is lifted: a plain tensor gets there
+    with pytest.raises(AssertionError):
+        mx.tile_scales(torch.zeros(128, 4, dtype=torch.uint8))
+
+
+def test_traced_encoding_replays_on_other_inputs(no_kernels):
+    """A trace of these functions holds the operations, not an empty tensor that a kernel once filled."""
+    g = torch.Generator().manual_seed(5)
+    x, y = torch.randn(128, 128, generator=g), torch.randn(128, 128, generator=g) * 40.0
+    sx, sy = (torch.randint(0, 256, (128, 8), generator=g, dtype=torch.uint8) for _ in range(2))
+    make_fx = torch.fx.experimental.proxy_tensor.make_fx
+    for got, want in zip(make_fx(mx.quantize_rows_mxfp8)(x)(y), mx._torch_quantize(y)):
+        assert torch.equal(got.reshape(-1), want)
+    for f in (make_fx(mx.tile_scales)(sx), torch.jit.trace(mx.tile_scales, sx, check_trace=False)):
+        assert torch.equal(f(sy), mx._torch_tile_scales(sy))
+    with pytest.raises(RuntimeError, match="aten::view"):            # torch.jit cannot record the view of e4m3 as bytes
+        torch.jit.trace(mx.quantize_rows_mxfp8, x, check_trace=False)
+
+
+@pytest.mark.parametrize("form", ["subclass", "mode", "functional", "functionalize", "zero", "jvp", "fake"])
+def test_encoding_of_tensors_that_are_not_plain_memory(form, no_kernels):
+    x = torch.randn(64, generator=torch.Generator().manual_seed(6))
+    want = mx._torch_quantize(x)
+    if form == "subclass":
+        got = mx.quantize_mxfp8(x.as_subclass(_Sub))
+    elif form == "mode":
+        with _Mode():
+            got = mx.quantize_mxfp8(x)
+    elif form == "functional":
+        got = mx.quantize_mxfp8(torch._to_functional_tensor(x))
+        want = tuple(map(torch.Tensor.tolist, want))
+        got = tuple(map(torch.Tensor.tolist, got))
+        assert got == want
+        return
+    elif form == "functionalize":
+        got = torch.func.functionalize(mx.quantize_mxfp8)(x)
+    elif form == "zero":
+        got, want = mx.quantize_mxfp8(torch._efficientzerotensor(64)), mx._torch_quantize(torch.zeros(64))
+    elif form == "jvp":
+        got, _ = torch.func.jvp(lambda t: tuple(o.float() for o in mx.quantize_mxfp8(t)), (x,), (torch.ones_like(x),))
+        want = tuple(o.float() for o in want)
+    else:
+        from torch._subclasses.fake_tensor import FakeTensorMode
+        with FakeTensorMode() as m:
+            d, s = mx.quantize_mxfp8(m.from_tensor(x))
+            assert tuple(d.shape) == (64,) and tuple(s.shape) == (2,)
+        return
+    assert all(torch.equal(a, b) for a, b in zip(got, want))

@@ -52,3 +52,14 @@ def test_tile_kernel_gives_the_bytes_of_the_torch_path(rows, kb):
     assert torch.equal(mx.tile_scales(s), mx._torch_tile_scales(s))
     off = torch.cat([s.new_zeros(1), s.reshape(-1)])[1:].view(rows, kb)      # not on a 4-byte boundary
     assert torch.equal(mx.tile_scales(off), mx._torch_tile_scales(s))
+
+
+def test_traced_encoding_replays_on_other_inputs():
+    """A recorded graph of the encoding on CUDA tensors holds the operations: it gives other inputs their own bytes."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, y = (torch.randn(128, 128, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    sx, sy = mx.quantize_rows_mxfp8(x)[1].repeat(1, 2), mx.quantize_rows_mxfp8(y * 40)[1].repeat(1, 2)
+    for got, want in zip(make_fx(mx.quantize_rows_mxfp8)(x)(y), mx._torch_quantize(y)):
+        assert torch.equal(got.reshape(-1), want)
+    assert torch.equal(torch.jit.trace(mx.tile_scales, sx, check_trace=False)(sy), mx._torch_tile_scales(sy))
