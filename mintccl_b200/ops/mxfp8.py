@@ -171,8 +171,8 @@ def tile_scales(scale: torch.Tensor) -> torch.Tensor:
     rows, kb = scale.shape
     if rows % 128 or kb % 4:
         raise ValueError("rows must be a multiple of 128 and K of 128")
-    if (scale.dtype is torch.uint8 and scale.is_contiguous() and scale.numel() and scale.data_ptr() % 4 == 0
-            and rows < 128 << 16 and _plain_cuda(scale)):
+    if (scale.dtype is torch.uint8 and _plain_cuda(scale) and scale.is_contiguous() and scale.numel()
+            and scale.data_ptr() % 4 == 0 and rows < 128 << 16):
         out = torch.empty(rows * kb, device=scale.device, dtype=torch.uint8)
         _on_device(scale, N.lib().mt_mxfp8_tile_scales, scale.data_ptr(), out.data_ptr(), rows, kb)
         return out

@@ -150,3 +150,12 @@ def test_encoding_of_tensors_that_are_not_plain_memory(form, no_kernels):
             assert tuple(d.shape) == (64,) and tuple(s.shape) == (2,)
         return
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("lifted", [False, True], ids=["cpu", "device_lifted"])
+def test_tile_scales_under_vmap(lifted, monkeypatch):
+    """A batched tensor has no address to ask for."""
+    if lifted:
+        monkeypatch.setattr(mx, "_plain_cuda", mx._is_plain)
+    s = torch.randint(0, 256, (3, 128, 8), generator=torch.Generator().manual_seed(7), dtype=torch.uint8)
+    assert torch.equal(torch.vmap(mx.tile_scales)(s), torch.stack([mx._torch_tile_scales(t) for t in s]))
