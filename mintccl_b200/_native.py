@@ -169,10 +169,17 @@ def u64_array(vals) -> "C.Array":
     return _U64s(*vals)
 
 
+_current_raw = None
+
+
 def raw_stream(device: int) -> int:
     """Handle of the current stream of ``device``.  The Stream object ``torch.cuda.current_stream`` builds for it costs
-    2 us, a fifth of the host time of a small launch."""
-    import torch
-    global raw_stream
-    raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda d: torch.cuda.current_stream(d).cuda_stream)
-    return raw_stream(device)
+    2 us, a fifth of the host time of a small launch.  A CPU tensor's device index is -1, which torch's raw query takes for
+    "the current device": it is refused here, before a kernel gets host addresses."""
+    global _current_raw
+    if device < 0:
+        raise ValueError("expected tensors on a CUDA device")
+    if _current_raw is None:
+        import torch
+        _current_raw = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda d: torch.cuda.current_stream(d).cuda_stream)
+    return _current_raw(device)

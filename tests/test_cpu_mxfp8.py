@@ -159,3 +159,16 @@ def test_tile_scales_under_vmap(lifted, monkeypatch):
         monkeypatch.setattr(mx, "_plain_cuda", mx._is_plain)
     s = torch.randint(0, 256, (3, 128, 8), generator=torch.Generator().manual_seed(7), dtype=torch.uint8)
     assert torch.equal(torch.vmap(mx.tile_scales)(s), torch.stack([mx._torch_tile_scales(t) for t in s]))
+
+
+def test_gemm_refuses_tensors_on_the_cpu(monkeypatch):
+    """Host addresses must not reach a kernel: the call ends before the native library is asked for anything."""
+    from mintccl_b200 import _native as N
+
+    def launch():
+        raise AssertionError("launched")
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda d: 0)
+    monkeypatch.setattr(N, "lib", launch)
+    d, s, w = torch.zeros(128, 128, dtype=torch.uint8), torch.zeros(128, 4, dtype=torch.uint8), torch.zeros(256, 128, dtype=torch.uint8)
+    with pytest.raises(ValueError, match="CUDA"):
+        mx.gemm_mxfp8(d, s, w, torch.zeros(256, 4, dtype=torch.uint8))
