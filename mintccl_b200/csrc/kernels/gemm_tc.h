@@ -12,8 +12,8 @@ enum GemmMode : int { MODE_PLAIN = 0, MODE_AG_GEMM = 1, MODE_GEMM_RS = 2 };
 // What the epilogue of a bf16 CTA-pair GEMM (plain, all-gather -> GEMM) does besides storing C.
 enum GemmEpi : int {
   EPI_NONE = 0,
-  EPI_SILU = 1,    // aux = silu(C), C as rounded
-  EPI_DSILU = 2,   // C = C * silu'(aux), aux read, C as rounded
+  EPI_SILU = 1,    // aux = silu(C), C as rounded (K-major operands)
+  EPI_DSILU = 2,   // C = C * silu'(aux), aux read, C as rounded (plain GEMM, B stored transposed)
 };
 
 // TMA descriptors, one set per local rank (index 0 outside single-GPU emulation).
@@ -43,7 +43,7 @@ struct GemmArgs {
   int32_t ta, tb;                      // CTA pairs, bf16: the operand is stored [K, M] / [K, N] (ta: plain GEMM only,
                                        // tb: plain and GEMM_RS); its map then has boxes of 64 columns x 64 K rows
   int32_t epi;                         // GemmEpi
-  int32_t wide_out;                    // rows of C (and aux) start on 32-byte boundaries
+  int32_t wide_out;                    // with epi: rows of C and aux start on 32-byte boundaries
   void* aux[MT_MAX_RANKS];             // second output (EPI_SILU) or input (EPI_DSILU), laid out like C
   int32_t raster;                      // plain GEMM: row blocks per group of the tile order (<= 1: row-major)
   uint64_t shard_off;                  // AG_GEMM pull: heap offset of every rank's own rows

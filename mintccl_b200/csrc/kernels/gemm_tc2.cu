@@ -71,8 +71,7 @@ struct Shape {
   static constexpr uint32_t SF_STAGE_BYTES = FP8 ? 512 * (1 + TILE_N / 128) : 0;
   static constexpr uint32_t RING = MODE == MODE_AG_GEMM ? fused::COMM_SLOTS * fused::COMM_PIECE : 0;   // comm CTAs reuse the stages
   static constexpr uint32_t OPERANDS = STAGES * (A_BYTES + B_PITCH) > RING ? STAGES * (A_BYTES + B_PITCH) : RING;
-  static constexpr uint32_t EPI = MODE == MODE_PLAIN ? 0 : EPI_BYTES;   // transpose of GEMM -> reduce-scatter; comm CTAs
-  static constexpr uint32_t SMEM = 1024 + OPERANDS + EPI + CTL_BYTES + STAGES * SF_STAGE_BYTES;
+  static constexpr uint32_t SMEM = 1024 + OPERANDS + EPI_BYTES + CTL_BYTES + STAGES * SF_STAGE_BYTES;
   static_assert(SMEM <= 232448, "shared memory of one CTA");
 };
 constexpr int MAX_STAGES = 10;
@@ -213,7 +212,8 @@ template <int MODE>
 constexpr int kMaps = MODE == MODE_PLAIN ? 1 : MT_MAX_RANKS;
 
 // TA, TB: the operand is stored transposed (compile-time: choosing descriptors in the issue loops cost 7 %).
-template <int MODE, bool FP8, int TILE_N, bool TA = false, bool TB = false>
+// EPI (GemmEpi): compile-time too, the code of the activations alone cost a plain 2048 x 4096 x 256 0.9 of 10.7 us.
+template <int MODE, bool FP8, int TILE_N, bool TA = false, bool TB = false, int EPI = EPI_NONE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_pair_kernel(const __grid_constant__ GemmMapsN<kMaps<MODE>> maps, const __grid_constant__ PairSfMapsN<kMaps<MODE>> sfmaps,
                      GemmArgs a) {
@@ -231,8 +231,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   uint8_t* sA = smem;
   uint8_t* sB = smem + STAGES * A_BYTES;
   uint8_t* sEpi = smem + S::OPERANDS;
-  Ctl* ctl = (Ctl*)(sEpi + S::EPI);
-  uint8_t* sSF = sEpi + S::EPI + CTL_BYTES;
+  Ctl* ctl = (Ctl*)(sEpi + EPI_BYTES);
+  uint8_t* sSF = sEpi + EPI_BYTES + CTL_BYTES;
   constexpr int BKE = FP8 ? 128 : 64;    // K elements per stage
   constexpr uint32_t ACC = FP8 && BN > 128 ? 1 : 2;  // accumulator buffers (MXFP8 keeps TMEM columns for the scales)
   const uint32_t cr = cluster_ctarank();
@@ -243,7 +243,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const uint64_t timeout_ns = a.timeout_ns;
 
   if (MODE == MODE_AG_GEMM && (int)blockIdx.x >= ngemm) {
-    fused::ag_comm_cta<FP8>(a, lr, (int)blockIdx.x - ngemm, nextra, smem, (fused::CommCtl*)(sEpi + S::EPI));
+    fused::ag_comm_cta<FP8>(a, lr, (int)blockIdx.x - ngemm, nextra, smem, (fused::CommCtl*)(sEpi + EPI_BYTES));
     return;
   }
   if (MODE == MODE_GEMM_RS && (int)blockIdx.x >= ngemm) {
@@ -277,7 +277,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);
   volatile int* abort_flag = &ctl->abort;
 
-  static_assert(!(TA || TB) || !FP8, "8-bit operands are K-major");
+  static_assert(!(TA || TB || EPI) || !FP8, "8-bit operands are K-major and have no activation");
   const int tiles = ((a.M + BM2 - 1) / BM2) * (a.N / BN);
   const int kblocks = a.K / BKE;
 
@@ -449,99 +449,90 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       const bool rows_out = MODE != MODE_PLAIN || tc_.mb * BM2 + (int)cr * BMC < a.M;   // M % 256 == 128: last peer has none
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN;
       const uint32_t acc_empty0 = map_to_cta(smem_u32(&ctl->acc_empty[as]), 0);
-      if constexpr (MODE == MODE_GEMM_RS) {
-        // Partial tiles go to a peer: whole 128-byte lines per store (a transpose through shared memory, 4 rows per pass
-        // of 8 lanes x 16 bytes), so that NVLink carries full packets.
-        auto store_block = [&](int cb) {
+      // Whole 128-byte lines per store: 64 columns of the warp's 32 rows go through shared memory and leave as 4 rows per
+      // pass of 8 lanes x 16 bytes (GEMM -> reduce-scatter: full NVLink packets).  Bound by the stores where K is small:
+      // 32-byte sectors straight from each lane's row took 68.4 us for an MXFP8 8192 x 14336 x 256, lines take 56.2, and
+      // 8192 x 4096 x 256 26.8 and 24.3 in bf16; from K = 1024 on, where the next tile's main loop hides the epilogue, both
+      // are within 2 %.  `n16`: 16-byte pieces per row (4: the last 32 of 224 columns).
+      // All 8 passes at once where the registers allow it (the fused MXFP8 kernels would spill; 4 cost the plain one 6 %).
+      auto lines_out = [&](int cb, const uint32_t* v, int n16) {
+        uint4* row = (uint4*)(stg + lane * EPI_PITCH);
 #pragma unroll
-          for (int p = 0; p < 8; ++p) {
-            const int rr = p * 4 + (lane >> 3), c16 = lane & 7;
-            const uint4 v = *(const uint4*)(stg + rr * EPI_PITCH + c16 * 16);
+        for (int j = 0; j < 8; ++j)
+          if (j < n16) row[j] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        __syncwarp();
+#pragma unroll(FP8 && MODE != MODE_PLAIN ? 4 : 8)
+        for (int p = 0; p < 8; ++p) {
+          const int rr = p * 4 + (lane >> 3), c16 = lane & 7;
+          if (c16 >= n16 || !rows_out) continue;
+          const uint4 x = *(const uint4*)(stg + rr * EPI_PITCH + c16 * 16);
+          uint8_t* g = dst + (uint64_t)rr * ld_bytes + cb * 128 + c16 * 16;
+          if (MODE == MODE_GEMM_RS) {
             u128 w;
-            w.x = (uint64_t)v.x | ((uint64_t)v.y << 32);
-            w.y = (uint64_t)v.z | ((uint64_t)v.w << 32);
-            store128_relaxed_sys(dst + (uint64_t)rr * ld_bytes + cb * 128 + c16 * 16, w);
+            w.x = (uint64_t)x.x | ((uint64_t)x.y << 32);
+            w.y = (uint64_t)x.z | ((uint64_t)x.w << 32);
+            store128_relaxed_sys(g, w);
+          } else {
+            *(uint4*)g = x;
           }
-        };
-        uint32_t pk[FP8 ? BN / 2 : 32];
-        auto stage_block = [&](int cb, const uint32_t* v) {
-          uint4* row = (uint4*)(stg + lane * EPI_PITCH);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) row[j] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          __syncwarp();
-          store_block(cb);
-          __syncwarp();
-        };
-        if constexpr (FP8) {
-          // single accumulator: drain it into registers (packed bf16) first and hand it back, then store
-#pragma unroll
-          for (int cb = 0; cb < BN / 64; ++cb) tmem_ld_pack64(taddr + cb * 64, pk + cb * 32);
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(acc_empty0);
-#pragma unroll
-          for (int cb = 0; cb < BN / 64; ++cb) stage_block(cb, pk + cb * 32);
-        } else {
-#pragma unroll 1
-          for (int cb = 0; cb < BN / 64; ++cb) {
-            tmem_ld_pack64(taddr + cb * 64, pk);
-            stage_block(cb, pk);
-          }
-          // accumulator drained: hand it back to the leader's MMA thread
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(acc_empty0);
         }
-      } else {
-        // Local output: every lane keeps the row it got from TMEM and stores it in whole 32-byte sectors.  The tensor
-        // cores read the operands, and TMA writes them, at the full rate of the shared memory (64 KiB per 512 cycles and
-        // k-block), so an epilogue that transposes through shared memory takes its cycles from the main loop; it also took
-        // 2 us at the end of a small problem, where nothing hides it.
-        uint8_t* row = dst + (uint64_t)lane * ld_bytes;
-        // activation fused into the epilogue: aux has C's layout (the work overlaps the next tile's main loop)
-        const int epi = FP8 ? EPI_NONE : a.epi;
-        uint8_t* aux = (uint8_t*)a.aux[lr] + (row - (uint8_t*)a.c[lr]);
-        const bool wide = a.wide_out != 0;
-        auto store32 = [&](int c32, const uint32_t* v) {   // 32 columns: 64 bytes
-          store_row64(row + c32 * 64, v, wide);
-        };
-        if constexpr (FP8) {
-          uint32_t pk[BN / 2];
+        __syncwarp();
+      };
+      // accumulator drained: hand it back to the leader's MMA thread
+      auto release_acc = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acc_empty0);
+      };
+      if constexpr (FP8) {
+        // drain the accumulator (256 columns: the only one) into registers (packed bf16) and hand it back, then store
+        uint32_t pk[BN / 2];
 #pragma unroll
-          for (int cb = 0; cb < BN / 64; ++cb) tmem_ld_pack64(taddr + cb * 64, pk + cb * 32);
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(acc_empty0);
-          if (rows_out) {
+        for (int cb = 0; cb < BN / 64; ++cb) tmem_ld_pack64(taddr + cb * 64, pk + cb * 32);
+        release_acc();
 #pragma unroll
-            for (int c = 0; c < BN / 32; ++c) store32(c, pk + c * 16);
-          }
-        } else {
+        for (int cb = 0; cb < BN / 64; ++cb) lines_out(cb, pk + cb * 32, 8);
+      } else if constexpr (EPI == EPI_NONE) {
 #pragma unroll 1
-          for (int c = 0; c < BN / 32; ++c) {
-            uint32_t r[32], v[16], h[16];
-            if (epi == EPI_DSILU && rows_out) load_row64(aux + c * 64, h, wide);
-            tmem_ld_32x32(taddr + c * 32, r);
-            tmem_ld_wait();
-            if (c == BN / 32 - 1) {
-              // accumulator drained: hand it back to the leader's MMA thread
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive_cluster(acc_empty0);
-            }
+        for (int cb = 0; cb < BN / 64; ++cb) {
+          uint32_t pk[32];
+          tmem_ld_pack64(taddr + cb * 64, pk);
+          lines_out(cb, pk, 8);
+        }
+        if (BN % 64) {
+          uint32_t r[32], pk[16];
+          tmem_ld_32x32(taddr + BN / 64 * 64, r);
+          tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-            if (!rows_out) continue;
-            if (epi == EPI_DSILU) {
+          for (int j = 0; j < 16; ++j) pk[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+          lines_out(BN / 64, pk, 4);
+        }
+        release_acc();
+      } else {
+        // activation fused into the epilogue (the work overlaps the next tile's main loop): aux has C's layout, and every
+        // lane keeps the row it got from TMEM and loads and stores it in whole 32-byte sectors
+        const bool wide = a.wide_out != 0;
+        uint8_t* row = dst + (uint64_t)lane * ld_bytes;
+        uint8_t* aux = (uint8_t*)a.aux[lr] + (row - (uint8_t*)a.c[lr]);
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t r[32], v[16], h[16];
+          if (EPI == EPI_DSILU && rows_out) load_row64(aux + c * 64, h, wide);
+          tmem_ld_32x32(taddr + c * 32, r);
+          tmem_ld_wait();
+          if (c == BN / 32 - 1) release_acc();
 #pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] = dsilu2(v[j], h[j]);
-            }
-            store32(c, v);
-            if (epi == EPI_SILU) {
+          for (int j = 0; j < 16; ++j) v[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+          if (!rows_out) continue;
+          if (EPI == EPI_DSILU) {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] = silu2(v[j]);
-              store_row64(aux + c * 64, v, wide);
-            }
+            for (int j = 0; j < 16; ++j) v[j] = dsilu2(v[j], h[j]);
+          }
+          store_row64(row + c * 64, v, wide);
+          if (EPI == EPI_SILU) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = silu2(v[j]);
+            store_row64(aux + c * 64, v, wide);
           }
         }
       }
@@ -576,28 +567,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
 }  // namespace pair
 
-// Operand forms of the bf16 kernels: 0 both K-major, 1 B stored transposed, 2 both stored transposed (plain GEMM only).
+// Forms of the bf16 kernels: operands as stored, and what the epilogue does.
+enum PairForm { FORM_NN = 0, FORM_TB, FORM_TA_TB, FORM_SILU, FORM_TB_DSILU, FORM_COUNT };
 struct PairKernel {
   const void* fn;
   uint32_t smem;
 };
-template <int MODE, bool FP8, int TILE_N, bool TA = false, bool TB = false>
+template <int MODE, bool FP8, int TILE_N, bool TA = false, bool TB = false, int EPI = EPI_NONE>
 static PairKernel pair_kernel() {
-  return {(const void*)pair::gemm_pair_kernel<MODE, FP8, TILE_N, TA, TB>, pair::Shape<MODE, FP8, TILE_N, TB>::SMEM};
+  return {(const void*)pair::gemm_pair_kernel<MODE, FP8, TILE_N, TA, TB, EPI>, pair::Shape<MODE, FP8, TILE_N, TB>::SMEM};
 }
-template <bool TA, bool TB>
+template <bool TA, bool TB, int EPI>
 static PairKernel plain_kernel(int bn) {
   switch (bn) {
-    case 256: return pair_kernel<MODE_PLAIN, false, 256, TA, TB>();
-    case 224: return pair_kernel<MODE_PLAIN, false, 224, TA, TB>();
-    case 128: return pair_kernel<MODE_PLAIN, false, 128, TA, TB>();
+    case 256: return pair_kernel<MODE_PLAIN, false, 256, TA, TB, EPI>();
+    case 224: return pair_kernel<MODE_PLAIN, false, 224, TA, TB, EPI>();
+    case 128: return pair_kernel<MODE_PLAIN, false, 128, TA, TB, EPI>();
+    case 64:
+      if constexpr (!TB) return pair_kernel<MODE_PLAIN, false, 64, TA, TB, EPI>();
+      return {nullptr, 0};
     default: return {nullptr, 0};
   }
 }
-static PairKernel pair_fn(int mode, bool fp8, int bn = 256, int form = 0) {
+static PairKernel pair_fn(int mode, bool fp8, int bn = 256, int form = FORM_NN) {
   const PairKernel none = {nullptr, 0};
   if (fp8) {
-    if (form) return none;
+    if (form != FORM_NN) return none;
     if (bn == 128) return mode == MODE_PLAIN ? pair_kernel<MODE_PLAIN, true, 128>() : none;
     if (bn != 256) return none;
     switch (mode) {
@@ -608,29 +603,44 @@ static PairKernel pair_fn(int mode, bool fp8, int bn = 256, int form = 0) {
     }
   }
   if (mode == MODE_PLAIN) {
-    if (form == 1) return plain_kernel<false, true>(bn);
-    if (form == 2) return plain_kernel<true, true>(bn);
-    return bn == 64 ? pair_kernel<MODE_PLAIN, false, 64>() : plain_kernel<false, false>(bn);
+    switch (form) {
+      case FORM_NN: return plain_kernel<false, false, EPI_NONE>(bn);
+      case FORM_TB: return plain_kernel<false, true, EPI_NONE>(bn);
+      case FORM_TA_TB: return plain_kernel<true, true, EPI_NONE>(bn);
+      case FORM_SILU: return plain_kernel<false, false, EPI_SILU>(bn);
+      case FORM_TB_DSILU: return plain_kernel<false, true, EPI_DSILU>(bn);
+      default: return none;
+    }
   }
-  if (mode == MODE_AG_GEMM && form == 0) {
-    if (bn == 224) return pair_kernel<MODE_AG_GEMM, false, 224>();
-    return bn == 256 ? pair_kernel<MODE_AG_GEMM, false, 256>() : none;
+  if (mode == MODE_AG_GEMM && (bn == 256 || bn == 224)) {
+    const bool wide = bn == 256;
+    if (form == FORM_NN) return wide ? pair_kernel<MODE_AG_GEMM, false, 256>() : pair_kernel<MODE_AG_GEMM, false, 224>();
+    if (form == FORM_SILU)
+      return wide ? pair_kernel<MODE_AG_GEMM, false, 256, false, false, EPI_SILU>()
+                  : pair_kernel<MODE_AG_GEMM, false, 224, false, false, EPI_SILU>();
+    return none;
   }
   if (mode == MODE_GEMM_RS && bn == 256) {
-    if (form == 1) return pair_kernel<MODE_GEMM_RS, false, 256, false, true>();
-    return form == 0 ? pair_kernel<MODE_GEMM_RS, false, 256>() : none;
+    if (form == FORM_TB) return pair_kernel<MODE_GEMM_RS, false, 256, false, true>();
+    return form == FORM_NN ? pair_kernel<MODE_GEMM_RS, false, 256>() : none;
   }
   return none;
+}
+// The form a launch asks for, -1 where there is no such kernel.
+static int form_of(const GemmArgs& a) {
+  if (a.ta) return a.tb && a.epi == EPI_NONE ? FORM_TA_TB : -1;
+  if (a.tb) return a.epi == EPI_NONE ? FORM_TB : (a.epi == EPI_DSILU ? FORM_TB_DSILU : -1);
+  return a.epi == EPI_NONE ? FORM_NN : (a.epi == EPI_SILU ? FORM_SILU : -1);
 }
 
 // Clusters of this kernel that the device can hold at once.  The kernel is persistent (cluster i takes tiles
 // i, i + n, ...), so a grid with more clusters than fit would run its tail after the rest has finished.
 int gemm_pair_max_clusters(int mode, bool fp8, int bn, int form) {
-  static int cached[72] = {};
+  static int cached[3 * 2 * 4 * FORM_COUNT] = {};
   const PairKernel k = pair_fn(mode, fp8, bn, form);
   if (!k.fn) return 0;
   const int width = bn == 256 ? 0 : (bn == 224 ? 1 : (bn == 128 ? 2 : 3));
-  int& slot = cached[((mode * 2 + (fp8 ? 1 : 0)) * 4 + width) * 3 + form];
+  int& slot = cached[((mode * 2 + (fp8 ? 1 : 0)) * 4 + width) * FORM_COUNT + form];
   if (slot > 0) return slot;
   if (cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem) != cudaSuccess) return 0;
   int dev = 0, sms = 148;
@@ -664,9 +674,9 @@ int gemm_pair_max_clusters(int mode, bool fp8, int bn, int form) {
 // Grid: 2 * nclusters GEMM CTAs followed by a.ncomm comm / reducer CTAs (even), times nlocal emulated ranks.
 cudaError_t launch_gemm_pair(int mode, const GemmMaps& maps, const PairSfMaps& sf, const GemmArgs& a, int nclusters,
                              int nlocal, cudaStream_t s, bool fp8, int bn) {
-  const int form = a.ta ? 2 : (a.tb ? 1 : 0);
-  const PairKernel k = pair_fn(mode, fp8, bn, form);
-  if (!k.fn || (a.ta && !a.tb)) return cudaErrorInvalidValue;
+  const int form = form_of(a);
+  const PairKernel k = form < 0 ? PairKernel{nullptr, 0} : pair_fn(mode, fp8, bn, form);
+  if (!k.fn) return cudaErrorInvalidValue;
   const int fit = gemm_pair_max_clusters(mode, fp8, bn, form);  // also sets the shared-memory attribute once
   if (fit <= 0) return cudaErrorInvalidValue;
   const int extra = mode == MODE_PLAIN ? 0 : a.ncomm;
