@@ -1,6 +1,7 @@
 // Host side of the tcgen05 GEMM kernels: TMA descriptors, argument checks, launches.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <string.h>
 
 #include <string>
@@ -109,8 +110,8 @@ static int raster_for(int /*M*/, int N, int K, int elem_bytes) {
   return b_bytes > 48e6 ? 16 : 1;
 }
 
-// GEMMs run on CTA pairs (gemm_tc2.cu); the fused kernels when a rank's rows are a multiple of 256, plain ones always (a last
-// block of 128 rows leaves its peer CTA idle).  MINTCCL_GEMM_PAIR=0: the single-CTA kernels of gemm_tc.cu.
+// GEMMs run on CTA pairs (gemm_tc2.cu); the fused kernels when a rank's rows are a multiple of 256, plain ones as gemm_plain
+// says.  MINTCCL_GEMM_PAIR=0: the single-CTA kernels of gemm_tc.cu.
 static int g_pair_mode = -1;
 static bool pair_on() {
   if (g_pair_mode < 0) {
@@ -145,7 +146,7 @@ static int pick_bn(int row_tiles, int N, int nclusters, bool fp8) {
 // the tile), and one k-block to drain the last accumulator.  So a problem with too few wide tiles for the chip takes
 // the widest ones that fill it.  Measured (us, 256 / 128 / 64 columns): 128 x 4096 x 1792 13.7 / 9.1 / 7.9,
 // 512 x 4096 x 1792 14.5 / 9.9 / 12.1, 1024 x 1792 x 4096 24.8 / 15.6 / 20.5, 2048 x 4096 x 2048 26.3 / 25.3 / 33.0.
-static int pick_plain_bn(int row_tiles, int N, int kblocks, int nclusters, bool fp8, bool tb) {
+static int pick_plain_bn(int row_tiles, int N, int kblocks, int nclusters, bool fp8, bool tb, long* cost_out = nullptr) {
   if (const int f = forced_bn(N, fp8, true, tb)) return f;
   const int wide = pick_wide(row_tiles, N, nclusters, fp8);
   if (nclusters < 1) return wide;
@@ -158,8 +159,17 @@ static int pick_plain_bn(int row_tiles, int N, int kblocks, int nclusters, bool 
     best = 128;
     c = cost(128, 11);
   }
-  if (!fp8 && !tb && cost(64, 8) < c) best = 64;
+  if (!fp8 && !tb && cost(64, 8) < c) {
+    best = 64;
+    c = cost(64, 8);
+  }
+  if (cost_out) *cost_out = c;
   return best;
+}
+// Clusters that `sms` SMs give a plain pair GEMM.
+static int pair_clusters(int sms, bool fp8) {
+  const int fit = mt::gemm_pair_max_clusters(mt::MODE_PLAIN, fp8), ncl = sms / 2;
+  return fit > 0 && ncl > fit ? fit : ncl;
 }
 
 static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N,
@@ -168,11 +178,7 @@ static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B
   int dev = 0;
   cudaGetDevice(&dev);
   const int row_tiles = (M + 255) / 256;
-  int ncl = (nctas > 0 ? nctas : sm_count(dev)) / 2;
-  {
-    const int fit = mt::gemm_pair_max_clusters(mt::MODE_PLAIN, fp8);
-    if (fit > 0 && ncl > fit) ncl = fit;
-  }
+  const int ncl = pair_clusters(nctas > 0 ? nctas : sm_count(dev), fp8);
   const int bn = pick_plain_bn(row_tiles, N, K / (fp8 ? 128 : 64), ncl, fp8, tb);
   mt::GemmMaps maps;
   mt::PairSfMaps sf;
@@ -210,6 +216,63 @@ static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B
   return 0;
 }
 
+// The same product on single CTAs (128 x 256 tiles), K-major operands.
+static int gemm_single(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N, int K,
+                       int ldc, int nctas, bool fp8, int stat) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  mt::GemmMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  if (make_map(&maps.a[0], A, M, K, kBM, fp8) || make_map(&maps.b[0], B, N, K, kBN, fp8)) return -1;
+  maps.a2[0] = maps.a[0];
+  mt::GemmArgs a;
+  memset(&a, 0, sizeof(a));
+  a.c[0] = C;
+  a.sfa[0] = sfa;
+  a.sfb[0] = sfb;
+  a.M = M;
+  a.N = N;
+  a.K = K;
+  a.ldc = ldc;
+  a.nranks = 1;
+  a.raster = raster_for(M, N, K, fp8 ? 1 : 2);
+  a.timeout_ns = 4000000000ull;
+  const int tiles = (M / kBM) * (N / kBN);
+  int grid = nctas > 0 ? nctas : sm_count(dev);
+  if (grid > tiles) grid = tiles;
+  cudaError_t e = mt::launch_gemm_tc(mt::MODE_PLAIN, maps, a, grid, 1, (cudaStream_t)stream, fp8);
+  if (e != cudaSuccess) return fail(std::string("gemm launch: ") + cudaGetErrorString(e));
+  mthost::stat_add(stat, (uint64_t)(2.0 * M * N * K));
+  return 0;
+}
+
+// C[M, ldc] = A[M, K] * B[N, K]^T, both K-major, on the kernel that suits the shape.  A last block of 128 rows leaves half a
+// pair idle, and 128-row tiles of single CTAs can need a wave less (1152 x 4096: 144 tiles on 148 SMs; pairs have 80 on 74
+// clusters).  In pick_plain_bn's unit (twice the tenths of a 256-column k-block) a wave of single CTAs costs 23 a k-block
+// and 5 (10 in MXFP8) for the drain; a lone bf16 wave 20.4 and 20 less, since nothing waits for its accumulator.  Of 418
+// shapes with 128 leftover rows (128 - 4224 x 256 - 14336, K = 256 - 8192, both types), timed on both kernels, four lose
+// 5 % by this choice and the others at most 3.  1152 x 4096 x 4096 takes 28.9 us (pairs 38.0), MXFP8 1152 x 4096 x 1024 10.4
+// (12.5), 640 x 4096 x 4096 26.8 (28.8); 2176 x 14336 x 1024 stays on pairs: 49.0, single CTAs 54.1.
+static long single_cost(int M, int N, int kblocks, int sms, bool fp8) {
+  const long waves = ((long)(M / kBM) * (N / kBN) + sms - 1) / sms;
+  if (waves == 1 && !fp8) return kblocks * 102L / 5 - 20;
+  return waves * (kblocks * 23L + (fp8 ? 10 : 5));
+}
+static int gemm_plain(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N, int K,
+                      int ldc, int nctas, bool fp8, int stat) {
+  bool single = !pair_on();
+  if (!single && M % 256 && !forced_bn(N, fp8, true, false)) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const int sms = nctas > 0 ? nctas : sm_count(dev), kblocks = K / (fp8 ? 128 : 64);
+    long pairs = LONG_MAX;   // fewer than two CTAs asked for: no pair
+    pick_plain_bn((M + 255) / 256, N, kblocks, pair_clusters(sms, fp8), fp8, false, &pairs);
+    single = single_cost(M, N, kblocks, sms, fp8) < pairs;
+  }
+  return single ? gemm_single(stream, A, sfa, B, sfb, C, M, N, K, ldc, nctas, fp8, stat)
+                : gemm_pair(stream, A, sfa, B, sfb, C, M, N, K, ldc, nctas, fp8, false, false, mt::EPI_NONE, nullptr, stat);
+}
+
 extern "C" {
 
 // 1 after a bounded wait of the CTA-pair GEMM expired (the result of that call is then invalid), 0 otherwise.
@@ -221,30 +284,7 @@ void mt_gemm_set_pair(int mode) { g_pair_mode = mode; }
 int mt_gemm(void* stream, const void* A, const void* B, void* C, int M, int N, int K, int ldc, int nctas) {
   if (check_shape(M, N, K, 1)) return -1;
   if (ldc < N || ldc % 8 || ((uintptr_t)C & 15)) return fail("C must be 16-byte aligned with ldc >= N, ldc % 8 == 0");
-  if (pair_on()) return gemm_pair(stream, A, nullptr, B, nullptr, C, M, N, K, ldc, nctas, false);
-  int dev = 0;
-  cudaGetDevice(&dev);
-  mt::GemmMaps maps;
-  memset(&maps, 0, sizeof(maps));
-  if (make_map(&maps.a[0], A, M, K, kBM) || make_map(&maps.b[0], B, N, K, kBN)) return -1;
-  maps.a2[0] = maps.a[0];
-  mt::GemmArgs a;
-  memset(&a, 0, sizeof(a));
-  a.c[0] = C;
-  a.M = M;
-  a.N = N;
-  a.K = K;
-  a.ldc = ldc;
-  a.nranks = 1;
-  a.raster = raster_for(M, N, K, 2);
-  a.timeout_ns = 4000000000ull;
-  const int tiles = (M / kBM) * (N / kBN);
-  int grid = nctas > 0 ? nctas : sm_count(dev);
-  if (grid > tiles) grid = tiles;
-  cudaError_t e = mt::launch_gemm_tc(mt::MODE_PLAIN, maps, a, grid, 1, (cudaStream_t)stream);
-  if (e != cudaSuccess) return fail(std::string("gemm launch: ") + cudaGetErrorString(e));
-  mthost::stat_add(mthost::ST_GEMM, (uint64_t)(2.0 * M * N * K));
-  return 0;
+  return gemm_plain(stream, A, nullptr, B, nullptr, C, M, N, K, ldc, nctas, false, mthost::ST_GEMM);
 }
 
 // C[M, N] = A * B in bf16 with fp32 accumulation, where either operand may be stored transposed: A as [K, M] (ta) or
@@ -272,32 +312,7 @@ int mt_gemm_mxfp8(void* stream, const void* A, const void* sfa, const void* B, c
   if (check_shape(M, N, K, 1) || K % 128) return fail("MXFP8 GEMM: M multiple of 128, N of 256, K of 128");
   if (ldc < N || ldc % 8 || ((uintptr_t)C & 15)) return fail("C must be 16-byte aligned with ldc >= N, ldc % 8 == 0");
   if (((uintptr_t)sfa | (uintptr_t)sfb) & 15) return fail("scale tensors must be 16-byte aligned");
-  if (pair_on()) return gemm_pair(stream, A, sfa, B, sfb, C, M, N, K, ldc, nctas, true);
-  int dev = 0;
-  cudaGetDevice(&dev);
-  mt::GemmMaps maps;
-  memset(&maps, 0, sizeof(maps));
-  if (make_map(&maps.a[0], A, M, K, kBM, true) || make_map(&maps.b[0], B, N, K, kBN, true)) return -1;
-  maps.a2[0] = maps.a[0];
-  mt::GemmArgs a;
-  memset(&a, 0, sizeof(a));
-  a.c[0] = C;
-  a.sfa[0] = sfa;
-  a.sfb[0] = sfb;
-  a.M = M;
-  a.N = N;
-  a.K = K;
-  a.ldc = ldc;
-  a.nranks = 1;
-  a.raster = raster_for(M, N, K, 1);
-  a.timeout_ns = 4000000000ull;
-  const int tiles = (M / kBM) * (N / kBN);
-  int grid = nctas > 0 ? nctas : sm_count(dev);
-  if (grid > tiles) grid = tiles;
-  cudaError_t e = mt::launch_gemm_tc(mt::MODE_PLAIN, maps, a, grid, 1, (cudaStream_t)stream, true);
-  if (e != cudaSuccess) return fail(std::string("mxfp8 gemm launch: ") + cudaGetErrorString(e));
-  mthost::stat_add(mthost::ST_GEMM_MXFP8, (uint64_t)(2.0 * M * N * K));
-  return 0;
+  return gemm_plain(stream, A, sfa, B, sfb, C, M, N, K, ldc, nctas, true, mthost::ST_GEMM_MXFP8);
 }
 
 static int fused_common(MtComm* c, mt::GemmArgs& a, int M, int N, int K, uint64_t flags_off, uint64_t epoch) {
@@ -342,8 +357,11 @@ static int ag_gemm_impl(MtComm* c, void* stream, const void* const* a_shard, con
   }
   if (n == 1 && (pair_on() || act)) {   // nothing to gather: the product itself
     if (((uintptr_t)C[0] & 15) || (fp8 && (((uintptr_t)sfa[0] | (uintptr_t)sfb[0]) & 15))) return fail("C and the scales must be 16-byte aligned");
-    return gemm_pair(stream, a_shard[0], fp8 ? sfa[0] : nullptr, B[0], fp8 ? sfb[0] : nullptr, C[0], M, N, K, ldc, nctas, fp8, false,
-                     false, a.epi, a.aux[0], mthost::ST_AG_GEMM);
+    if (!act)
+      return gemm_plain(stream, a_shard[0], fp8 ? sfa[0] : nullptr, B[0], fp8 ? sfb[0] : nullptr, C[0], M, N, K, ldc, nctas, fp8,
+                        mthost::ST_AG_GEMM);
+    return gemm_pair(stream, a_shard[0], nullptr, B[0], nullptr, C[0], M, N, K, ldc, nctas, false, false, false, a.epi, a.aux[0],
+                     mthost::ST_AG_GEMM);
   }
   if (n == 1) ncomm = 0;
   else if (ncomm < 1 || ncomm > 64) return fail("ncomm out of range");
@@ -441,11 +459,11 @@ static int gemm_rs_impl(MtComm* c, void* stream, const void* const* A, const voi
     // 128 us with them, 83 without).  The sum of one bf16 partial tile is that tile, so the bytes are the same.
     if ((uintptr_t)out[0] & 15) return fail("out must be 16-byte aligned");
     if (fp8 && (((uintptr_t)sfa[0] | (uintptr_t)sfb[0]) & 15)) return fail("scale tensors must be 16-byte aligned");
-    if (tb || pair_on())
-      return gemm_pair(stream, A[0], fp8 ? sfa[0] : nullptr, B[0], fp8 ? sfb[0] : nullptr, out[0], M, N, K, N, nctas, fp8, false, tb,
-                       mt::EPI_NONE, nullptr, mthost::ST_GEMM_RS);
-    return fp8 ? mt_gemm_mxfp8(stream, A[0], sfa[0], B[0], sfb[0], out[0], M, N, K, N, nctas)
-               : mt_gemm(stream, A[0], B[0], out[0], M, N, K, N, nctas);
+    if (tb)
+      return gemm_pair(stream, A[0], nullptr, B[0], nullptr, out[0], M, N, K, N, nctas, false, false, true, mt::EPI_NONE, nullptr,
+                       mthost::ST_GEMM_RS);
+    return gemm_plain(stream, A[0], fp8 ? sfa[0] : nullptr, B[0], fp8 ? sfb[0] : nullptr, out[0], M, N, K, N, nctas, fp8,
+                      mthost::ST_GEMM_RS);
   }
   if (tb && !use_pair(M / c->nranks)) return fail("a transposed B needs rows per rank that are a multiple of 256");
   int grid = nctas > 0 ? nctas : sm_count(c->device);

@@ -299,3 +299,22 @@ def test_narrow_tiles_give_the_bits_of_wide_ones(shape, bn, form, monkeypatch):
     if form == "plain":
         close(out, ref_mm(a, w), K)
     assert torch.equal(out, wide) and torch.equal(chosen, wide)
+
+
+@pytest.mark.parametrize("shape", [(1152, 4096, 128), (1152, 4096, 1024), (128, 14336, 512), (2176, 1792, 256), (4224, 4096, 512)])
+def test_128_leftover_rows_give_the_bits_of_pairs(shape, monkeypatch):
+    """Shapes on both sides of the rule that sends a problem with 128 leftover rows to single CTAs (all but the last)."""
+    from mintccl_b200.ops import gemm as G
+    from mintccl_b200.ops import mxfp8 as mx
+    M, Nn, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + Nn + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(Nn, K, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    qa, qw = mx.quantize_rows_mxfp8(a), mx.quantize_rows_mxfp8(w)
+    for call in (lambda **k: G.gemm(a, w, **k), lambda **k: mx.gemm_mxfp8(*qa, *qw, **k)):
+        chosen, few = call(), call(nctas=1)
+        monkeypatch.setenv("MINTCCL_GEMM_BN", "256")
+        pairs = call()
+        monkeypatch.delenv("MINTCCL_GEMM_BN")
+        assert torch.equal(chosen, pairs) and torch.equal(few, pairs)
+    close(G.gemm(a, w), ref_mm(a, w), K)
