@@ -280,10 +280,29 @@ __device__ __forceinline__ u128 shift_bytes(u128 cur, u128 next, uint32_t s) {
   return o;
 }
 
+// At most kFewBytes * NTHREADS bytes, wherever they lie: one round trip with all bytes of a thread in flight.  Putting
+// vectors together (copy_range_shifted) takes a warp 0.7 us of dependent instructions more, for each peer in turn: an
+// all-to-all of 101-byte rows on 8 emulated ranks takes 23.4 us that way and 17.5 this way, of 1001-byte ones 24.7 and 18.8.
+constexpr int kFewBytes = 4;
+template <int NTHREADS>
+__device__ __noinline__ void copy_few_bytes(const uint8_t* src, uint8_t* dst, uint32_t nbytes) {
+  uint8_t v[kFewBytes];
+#pragma unroll
+  for (int k = 0; k < kFewBytes; ++k) {
+    const uint32_t o = threadIdx.x + k * NTHREADS;
+    if (o < nbytes) v[k] = *reinterpret_cast<const volatile uint8_t*>(src + o);
+  }
+#pragma unroll
+  for (int k = 0; k < kFewBytes; ++k) {
+    const uint32_t o = threadIdx.x + k * NTHREADS;
+    if (o < nbytes) *reinterpret_cast<volatile uint8_t*>(dst + o) = v[k];
+  }
+}
+
 // The copy when src and dst are not both on 16-byte boundaries (rows of an all-gather whose size is no multiple of 16):
 // aligned 16-byte loads and stores all the same.  Where the two differ in their offset, a lane's vector is put together
 // from its own aligned block and its neighbour's (one shuffle, every block is read once); no block outside
-// [src, src + nbytes) is touched, the edges (under 48 bytes in all) go byte by byte.  Bytewise copies took 97 - 110 us
+// [src, src + nbytes) is touched, the edges go byte by byte.  Bytewise copies took 97 - 110 us
 // for an all-gather of four 2 MB shards on four emulated ranks (0.4 TB/s), this one 24 - 27 with the launch.
 template <int NTHREADS, bool REMOTE_SRC, bool REMOTE_DST>
 __device__ __forceinline__ void copy_range_shifted(const uint8_t* src, uint8_t* dst, uint64_t nbytes) {
@@ -295,42 +314,41 @@ __device__ __forceinline__ void copy_range_shifted(const uint8_t* src, uint8_t* 
   // output i = bytes s .. s + 15 of blocks i, i + 1 of the source; with s == 0 block i alone
   const uint64_t blocks = nbytes + s >= head ? (nbytes + s - head) >> 4 : 0;
   const uint64_t nvec = s == 0 ? blocks : (blocks > 0 ? blocks - 1 : 0);
+  // The edges, bytes [0, head) and [done, nbytes): at most 61, one to a thread, loaded first and stored last.
+  static_assert(NTHREADS >= 64, "an edge byte per thread");
+  const uint64_t done = head + (nvec << 4), o = threadIdx.x;
+  const bool edge = o < head + (nbytes - done);
+  const uint64_t eb = o < head ? o : done + (o - head);
+  uint8_t ev = 0;
+  if (edge) ev = *reinterpret_cast<const volatile uint8_t*>(src + eb);
   const uint8_t* a = src + head - s;
   auto load = [&](uint64_t i) { return REMOTE_SRC ? load128_relaxed_sys(a + (i << 4)) : load128_stream(a + (i << 4)); };
-  if (nvec > 0) {
-    for (uint64_t base = (uint64_t)(threadIdx.x >> 5) * (32 * kU); base < nvec; base += (uint64_t)NTHREADS * kU) {
-      u128 v[kU + 1];
+  for (uint64_t base = (uint64_t)(threadIdx.x >> 5) * (32 * kU); base < nvec; base += (uint64_t)NTHREADS * kU) {
+    u128 v[kU + 1];
 #pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const uint64_t i = base + u * 32 + lane;
-        if (i < blocks) v[u] = load(i);
+    for (int u = 0; u < kU; ++u) {
+      const uint64_t i = base + u * 32 + lane;
+      if (i < blocks) v[u] = load(i);
+    }
+    if (s != 0 && base + kU * 32 < blocks) v[kU] = load(base + kU * 32);   // the block after the warp's last one
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint64_t i = base + u * 32 + lane;
+      u128 o16 = v[u];
+      if (s != 0) {
+        const u128 give = lane == 0 ? v[u + 1] : v[u];
+        u128 next;
+        next.x = __shfl_sync(0xffffffffu, give.x, (lane + 1) & 31);
+        next.y = __shfl_sync(0xffffffffu, give.y, (lane + 1) & 31);
+        o16 = shift_bytes(o16, next, s);
       }
-      if (s != 0 && base + kU * 32 < blocks) v[kU] = load(base + kU * 32);   // the block after the warp's last one
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const uint64_t i = base + u * 32 + lane;
-        u128 o = v[u];
-        if (s != 0) {
-          const u128 give = lane == 0 ? v[u + 1] : v[u];
-          u128 next;
-          next.x = __shfl_sync(0xffffffffu, give.x, (lane + 1) & 31);
-          next.y = __shfl_sync(0xffffffffu, give.y, (lane + 1) & 31);
-          o = shift_bytes(o, next, s);
-        }
-        if (i < nvec) {
-          if (REMOTE_DST) store128_relaxed_sys(dst + head + (i << 4), o);
-          else *reinterpret_cast<u128*>(dst + head + (i << 4)) = o;
-        }
+      if (i < nvec) {
+        if (REMOTE_DST) store128_relaxed_sys(dst + head + (i << 4), o16);
+        else *reinterpret_cast<u128*>(dst + head + (i << 4)) = o16;
       }
     }
-  } else {
-    head = 0;
   }
-  const uint64_t done = head + (nvec << 4);        // bytes [0, head) and [done, nbytes) are left
-  for (uint64_t o = threadIdx.x; o < head + (nbytes - done); o += NTHREADS) {
-    const uint64_t b = o < head ? o : done + (o - head);
-    *reinterpret_cast<volatile uint8_t*>(dst + b) = *reinterpret_cast<const volatile uint8_t*>(src + b);
-  }
+  if (edge) *reinterpret_cast<volatile uint8_t*>(dst + eb) = ev;
 }
 
 // Copy [lo, hi) bytes from src to dst with 16-byte vectors (+ byte tail).  REMOTE_SRC / REMOTE_DST
@@ -357,6 +375,8 @@ __device__ __forceinline__ void copy_range(const uint8_t* src, uint8_t* dst, uin
     }
     for (uint64_t o = (nvec << 4) + threadIdx.x; o < nbytes; o += NTHREADS)
       *reinterpret_cast<volatile uint8_t*>(dst + o) = *reinterpret_cast<const volatile uint8_t*>(src + o);
+  } else if (nbytes <= (uint64_t)kFewBytes * NTHREADS) {
+    copy_few_bytes<NTHREADS>(src, dst, (uint32_t)nbytes);
   } else {
     copy_range_shifted<NTHREADS, REMOTE_SRC, REMOTE_DST>(src, dst, nbytes);
   }

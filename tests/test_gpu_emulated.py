@@ -627,7 +627,7 @@ def test_reduce_with_a_summing_root(n, numel, algo="direct2"):
 
 
 @pytest.mark.parametrize("algo", ["direct", "pull", "bulk"])
-@pytest.mark.parametrize("nbytes", [1, 15, 17, 31, 47, 48, 49, 2047, 8193, 100_003])
+@pytest.mark.parametrize("nbytes", [1, 15, 17, 31, 47, 48, 49, 2047, 8193, 32_767, 32_785, 33_001, 100_003])
 def test_allgather_of_rows_off_the_16_byte_grid(algo, nbytes):
     """Rows whose size is no multiple of 16 and contributions that start anywhere: every pair of offsets of source and
     destination, sizes around the vector, the warp's chunk and the CTA's slice.  Bytes outside the rows stay as they are."""
