@@ -140,6 +140,7 @@ def lib():
     sig("mt_mxfp8_quantize", i32, vp, i32, vp, vp, vp, u64)
     sig("mt_mxfp8_tile_scales", i32, vp, vp, vp, u64, u64)
     sig("mt_test_wait_timeout", i32, vp, vp)
+    sig("mt_test_one_rank_args", i32, u64, vp, u64, C.POINTER(u64))
     sig("mt_find_ring", i32, C.POINTER(C.c_double), i32, ip)
     sig("mt_find_route", i32, C.POINTER(C.c_double), i32, i32, i32, ip)
     sig("mt_topo_probe", i32, i32, C.POINTER(C.c_double), i32, u64)

@@ -172,9 +172,33 @@ static int pair_clusters(int sms, bool fp8) {
   return fit > 0 && ncl > fit ? fit : ncl;
 }
 
+// How long a wait inside a product may take, and the status record that learns of one that took longer: those of the
+// communicator whose one-rank plan it stands in for; by default 4 s and none (mt_gemm_pair_error).
+struct Waits {
+  uint64_t timeout_ns = 4000000000ull;
+  void* status = nullptr;
+  int rank = 0;
+};
+static Waits waits_of(const mt::GemmArgs& plan) { return {plan.timeout_ns, plan.status[0], plan.rank[0]}; }
+
+static mt::GemmArgs product_args(void* C, int M, int N, int K, int ldc, const Waits& waits) {
+  mt::GemmArgs a;
+  memset(&a, 0, sizeof(a));
+  a.c[0] = C;
+  a.M = M;
+  a.N = N;
+  a.K = K;
+  a.ldc = ldc;
+  a.nranks = 1;
+  a.timeout_ns = waits.timeout_ns;
+  a.status[0] = waits.status;
+  a.rank[0] = waits.rank;
+  return a;
+}
+
 static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N,
-                     int K, int ldc, int nctas, bool fp8, bool ta = false, bool tb = false, int epi = mt::EPI_NONE,
-                     void* aux = nullptr, int stat = -1) {
+                     int K, int ldc, int nctas, bool fp8, int stat, const Waits& waits, bool ta = false, bool tb = false,
+                     int epi = mt::EPI_NONE, void* aux = nullptr) {
   int dev = 0;
   cudaGetDevice(&dev);
   const int row_tiles = (M + 255) / 256;
@@ -192,51 +216,35 @@ static int gemm_pair(void* stream, const void* A, const void* sfa, const void* B
         make_sf_map(&sf.sfb[0], sfb, (uint64_t)(N / 128) * (K / 128)))
       return -1;
   }
-  mt::GemmArgs a;
-  memset(&a, 0, sizeof(a));
-  a.c[0] = C;
-  a.M = M;
-  a.N = N;
-  a.K = K;
-  a.ldc = ldc;
-  a.nranks = 1;
+  mt::GemmArgs a = product_args(C, M, N, K, ldc, waits);
   a.ta = ta;
   a.tb = tb;
   a.epi = epi;
   a.aux[0] = aux;
   a.raster = raster_for(M, N, K, fp8 ? 1 : 2) / 2;
-  a.timeout_ns = 4000000000ull;
   const int tiles = row_tiles * (N / bn);
   int nclusters = (nctas > 0 ? nctas : sm_count(dev)) / 2;
   if (nclusters > tiles) nclusters = tiles;
   if (nclusters < 1) nclusters = 1;
   cudaError_t e = mt::launch_gemm_pair(mt::MODE_PLAIN, maps, sf, a, nclusters, 1, (cudaStream_t)stream, fp8, bn);
   if (e != cudaSuccess) return fail(std::string("pair gemm launch: ") + cudaGetErrorString(e));
-  mthost::stat_add(stat >= 0 ? stat : (fp8 ? mthost::ST_GEMM_MXFP8 : mthost::ST_GEMM), (uint64_t)(2.0 * M * N * K));
+  mthost::stat_add(stat, (uint64_t)(2.0 * M * N * K));
   return 0;
 }
 
 // The same product on single CTAs (128 x 256 tiles), K-major operands.
 static int gemm_single(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N, int K,
-                       int ldc, int nctas, bool fp8, int stat) {
+                       int ldc, int nctas, bool fp8, int stat, const Waits& waits) {
   int dev = 0;
   cudaGetDevice(&dev);
   mt::GemmMaps maps;
   memset(&maps, 0, sizeof(maps));
   if (make_map(&maps.a[0], A, M, K, kBM, fp8) || make_map(&maps.b[0], B, N, K, kBN, fp8)) return -1;
   maps.a2[0] = maps.a[0];
-  mt::GemmArgs a;
-  memset(&a, 0, sizeof(a));
-  a.c[0] = C;
+  mt::GemmArgs a = product_args(C, M, N, K, ldc, waits);
   a.sfa[0] = sfa;
   a.sfb[0] = sfb;
-  a.M = M;
-  a.N = N;
-  a.K = K;
-  a.ldc = ldc;
-  a.nranks = 1;
   a.raster = raster_for(M, N, K, fp8 ? 1 : 2);
-  a.timeout_ns = 4000000000ull;
   const int tiles = (M / kBM) * (N / kBN);
   int grid = nctas > 0 ? nctas : sm_count(dev);
   if (grid > tiles) grid = tiles;
@@ -259,7 +267,7 @@ static long single_cost(int M, int N, int kblocks, int sms, bool fp8) {
   return waves * (kblocks * 23L + (fp8 ? 10 : 5));
 }
 static int gemm_plain(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N, int K,
-                      int ldc, int nctas, bool fp8, int stat) {
+                      int ldc, int nctas, bool fp8, int stat, const Waits& waits = Waits()) {
   bool single = !pair_on();
   if (!single && M % 256 && !forced_bn(N, fp8, true, false)) {
     int dev = 0;
@@ -269,8 +277,8 @@ static int gemm_plain(void* stream, const void* A, const void* sfa, const void* 
     pick_plain_bn((M + 255) / 256, N, kblocks, pair_clusters(sms, fp8), fp8, false, &pairs);
     single = single_cost(M, N, kblocks, sms, fp8) < pairs;
   }
-  return single ? gemm_single(stream, A, sfa, B, sfb, C, M, N, K, ldc, nctas, fp8, stat)
-                : gemm_pair(stream, A, sfa, B, sfb, C, M, N, K, ldc, nctas, fp8, false, false, mt::EPI_NONE, nullptr, stat);
+  return single ? gemm_single(stream, A, sfa, B, sfb, C, M, N, K, ldc, nctas, fp8, stat, waits)
+                : gemm_pair(stream, A, sfa, B, sfb, C, M, N, K, ldc, nctas, fp8, stat, waits);
 }
 
 extern "C" {
@@ -292,13 +300,13 @@ int mt_gemm(void* stream, const void* A, const void* B, void* C, int M, int N, i
 int mt_gemm_t(void* stream, const void* A, const void* B, void* C, int M, int N, int K, int ta, int tb) {
   if (check_shape(M, N, K, 1)) return -1;
   if ((uintptr_t)C & 15) return fail("C must be 16-byte aligned");
-  return gemm_pair(stream, A, nullptr, B, nullptr, C, M, N, K, N, 0, false, ta != 0, tb != 0);
+  return gemm_pair(stream, A, nullptr, B, nullptr, C, M, N, K, N, 0, false, mthost::ST_GEMM, Waits(), ta != 0, tb != 0);
 }
 // C[M, N] = (A[M, K] * B[K, N]) * silu'(H[M, N]): the gradient through silu and the layer behind it.
 int mt_gemm_dsilu(void* stream, const void* A, const void* B, const void* H, void* C, int M, int N, int K) {
   if (check_shape(M, N, K, 1)) return -1;
   if (((uintptr_t)C | (uintptr_t)H) & 15) return fail("C and H must be 16-byte aligned");
-  return gemm_pair(stream, A, nullptr, B, nullptr, C, M, N, K, N, 0, false, false, true, mt::EPI_DSILU, (void*)H);
+  return gemm_pair(stream, A, nullptr, B, nullptr, C, M, N, K, N, 0, false, mthost::ST_GEMM, Waits(), false, true, mt::EPI_DSILU, (void*)H);
 }
 // Do problems of `rows` rows per rank run on CTA pairs (the kernels that take a transposed B)?
 int mt_gemm_uses_pair(int rows) { return use_pair(rows) ? 1 : 0; }
@@ -335,6 +343,22 @@ static int fused_common(MtComm* c, mt::GemmArgs& a, int M, int N, int K, uint64_
   return 0;
 }
 
+// Host-side check of what a one-rank plan's product is launched with: out = {time limit, status record, rank}.
+int mt_test_one_rank_args(uint64_t timeout_ns, void* heap, uint64_t status_off, uint64_t* out) {
+  MtComm c;
+  c.timeout_ns = timeout_ns;
+  c.heap[0][0] = (uint8_t*)heap;
+  c.L.status_off = status_off;
+  c.d_comms = (MtDevComm*)heap;
+  mt::GemmArgs plan;
+  if (fused_common(&c, plan, 128, 256, 64, 0, 1)) return -1;
+  const mt::GemmArgs a = product_args(nullptr, 128, 256, 64, 256, waits_of(plan));
+  out[0] = a.timeout_ns;
+  out[1] = (uint64_t)(uintptr_t)a.status[0];
+  out[2] = (uint64_t)a.rank[0];
+  return 0;
+}
+
 // C[M, ldc] = allgather(a_shard)[M, K] * B[N, K]^T.  `gather_off`: symmetric buffer of M * K bf16;
 // `flags_off`: symmetric u64 counters [ranks][M / ranks / 128], zero before the first call; `epoch`: 1 on the
 // first call on these counters, then 2, 3, ...; `ncomm` must not change between calls on the same counters.
@@ -359,9 +383,9 @@ static int ag_gemm_impl(MtComm* c, void* stream, const void* const* a_shard, con
     if (((uintptr_t)C[0] & 15) || (fp8 && (((uintptr_t)sfa[0] | (uintptr_t)sfb[0]) & 15))) return fail("C and the scales must be 16-byte aligned");
     if (!act)
       return gemm_plain(stream, a_shard[0], fp8 ? sfa[0] : nullptr, B[0], fp8 ? sfb[0] : nullptr, C[0], M, N, K, ldc, nctas, fp8,
-                        mthost::ST_AG_GEMM);
-    return gemm_pair(stream, a_shard[0], nullptr, B[0], nullptr, C[0], M, N, K, ldc, nctas, false, false, false, a.epi, a.aux[0],
-                     mthost::ST_AG_GEMM);
+                        mthost::ST_AG_GEMM, waits_of(a));
+    return gemm_pair(stream, a_shard[0], nullptr, B[0], nullptr, C[0], M, N, K, ldc, nctas, false, mthost::ST_AG_GEMM, waits_of(a),
+                     false, false, a.epi, a.aux[0]);
   }
   if (n == 1) ncomm = 0;
   else if (ncomm < 1 || ncomm > 64) return fail("ncomm out of range");
@@ -460,10 +484,10 @@ static int gemm_rs_impl(MtComm* c, void* stream, const void* const* A, const voi
     if ((uintptr_t)out[0] & 15) return fail("out must be 16-byte aligned");
     if (fp8 && (((uintptr_t)sfa[0] | (uintptr_t)sfb[0]) & 15)) return fail("scale tensors must be 16-byte aligned");
     if (tb)
-      return gemm_pair(stream, A[0], nullptr, B[0], nullptr, out[0], M, N, K, N, nctas, false, false, true, mt::EPI_NONE, nullptr,
-                       mthost::ST_GEMM_RS);
+      return gemm_pair(stream, A[0], nullptr, B[0], nullptr, out[0], M, N, K, N, nctas, false, mthost::ST_GEMM_RS, waits_of(a),
+                       false, true);
     return gemm_plain(stream, A[0], fp8 ? sfa[0] : nullptr, B[0], fp8 ? sfb[0] : nullptr, out[0], M, N, K, N, nctas, fp8,
-                      mthost::ST_GEMM_RS);
+                      mthost::ST_GEMM_RS, waits_of(a));
   }
   if (tb && !use_pair(M / c->nranks)) return fail("a transposed B needs rows per rank that are a multiple of 256");
   int grid = nctas > 0 ? nctas : sm_count(c->device);

@@ -551,7 +551,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     // tell the peer (it would notice by itself after its own time limit) and the host
     st_cluster_u32(map_to_cta(smem_u32(&ctl->abort), cr ^ 1), 1u);
     atomicExch(&g_pair_error, 1);
-    if (MODE != MODE_PLAIN) fused::gemm_report(a, lr, MT_WHERE_GEMM_FLAG);
+    fused::gemm_report(a, lr, MT_WHERE_GEMM_FLAG);   // the plain GEMM has no status record, a one-rank plan does
   }
   cluster_sync_all();  // neither CTA leaves, or frees TMEM, while the other may still signal into it
   if (warp == 1) {

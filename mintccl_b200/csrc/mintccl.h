@@ -157,6 +157,8 @@ int mt_mxfp8_tile_scales(void* stream, const void* in, void* out, uint64_t rows,
 
 // ---- device-wait self test: a wait nothing satisfies must time out and report, not hang -----------
 int mt_test_wait_timeout(MtComm* c, void* stream);
+// what the product of a one-rank plan is launched with (no GPU): out = {time limit in ns, status record, rank}
+int mt_test_one_rank_args(uint64_t timeout_ns, void* heap, uint64_t status_off, uint64_t* out);
 
 // ---- host model of the fused GEMM + collective protocols (threads and atomics, no GPU; sim/sim_fused.cpp) ----
 // op: 0 all-gather -> GEMM, 1 GEMM -> reduce-scatter.  Returns 0 ok, 1 data of another call was read, 2 a wait gave

@@ -460,3 +460,12 @@ def test_tuning_table_ignores_noise_and_keeps_memory_kinds_apart():
     assert t.lookup("allgather", 8, 1 << 28, True) == ("ring", 64)
     assert t.lookup("allgather", 8, 1 << 26, False) == ("direct", 64)
     assert t.lookup("allgather", 8, 1 << 28, False) is None
+
+
+def test_one_rank_plans_keep_the_limit_and_the_status_record_of_their_communicator():
+    """The product that stands in for a one-rank fused plan reports an expired wait where ``comm.check()`` looks."""
+    import ctypes as C
+    heap, out = C.create_string_buffer(4096), (C.c_uint64 * 3)()
+    base = C.addressof(heap)
+    assert N.lib().mt_test_one_rank_args(1_234_567, base, 640, out) == 0
+    assert list(out) == [1_234_567, base + 640, 0]
