@@ -379,7 +379,9 @@ static int ag_gemm_impl(MtComm* c, void* stream, const void* const* a_shard, con
     a.epi = mt::EPI_SILU;
     if (n > 1 && (!use_pair(M / n) || comm_mode == 2)) return fail("the fused activation runs on CTA pairs");
   }
+  if (comm_mode < 0 || comm_mode > 3) return fail("comm_mode must be 0, 1, 2 or 3");
   if (n == 1 && (pair_on() || act)) {   // nothing to gather: the product itself
+    if (nctas == 1 && use_pair(M) && comm_mode != 2) return fail("not enough CTAs for the requested comm CTAs");
     if (((uintptr_t)C[0] & 15) || (fp8 && (((uintptr_t)sfa[0] | (uintptr_t)sfb[0]) & 15))) return fail("C and the scales must be 16-byte aligned");
     if (!act)
       return gemm_plain(stream, a_shard[0], fp8 ? sfa[0] : nullptr, B[0], fp8 ? sfb[0] : nullptr, C[0], M, N, K, ldc, nctas, fp8,
@@ -400,7 +402,6 @@ static int ag_gemm_impl(MtComm* c, void* stream, const void* const* a_shard, con
   if (n > 1 && (comm_split < 1 || comm_split > ncomm)) return fail("comm_split must be in [1, ncomm]");
   a.comm_split = n > 1 ? comm_split : 1;
   a.shard_off = shard_off;
-  if (comm_mode < 0 || comm_mode > 3) return fail("comm_mode must be 0, 1, 2 or 3");
   mt::GemmMaps maps;
   memset(&maps, 0, sizeof(maps));
   for (int lr = 0; lr < c->nlocal; ++lr) {
@@ -478,6 +479,9 @@ static int gemm_rs_impl(MtComm* c, void* stream, const void* const* A, const voi
   mt::GemmArgs a;
   if (fp8 && K % 128) return fail("MXFP8: K must be a multiple of 128");
   if (fused_common(c, a, M, N, K, flags_off, epoch)) return -1;
+  int grid = nctas > 0 ? nctas : sm_count(c->device);
+  if (c->emulated && grid * c->nlocal > sm_count(c->device)) grid = sm_count(c->device) / c->nlocal;
+  if (nred < 0 || nred >= grid || (use_pair(M / c->nranks) && grid - ((nred + 1) & ~1) < 2)) return fail("nred out of range");
   if (c->nranks == 1) {
     // nothing to reduce: the product itself, without the staging area and the reducers' pass over it (8192 x 4096 x 1792:
     // 128 us with them, 83 without).  The sum of one bf16 partial tile is that tile, so the bytes are the same.
@@ -490,9 +494,6 @@ static int gemm_rs_impl(MtComm* c, void* stream, const void* const* A, const voi
                       mthost::ST_GEMM_RS, waits_of(a));
   }
   if (tb && !use_pair(M / c->nranks)) return fail("a transposed B needs rows per rank that are a multiple of 256");
-  int grid = nctas > 0 ? nctas : sm_count(c->device);
-  if (c->emulated && grid * c->nlocal > sm_count(c->device)) grid = sm_count(c->device) / c->nlocal;
-  if (nred < 0 || nred >= grid) return fail("nred out of range");
   a.ncomm = nred;
   a.ldc = N;
   a.stage_off = stage_off + (epoch & 1) * (uint64_t)M * N * 2;
@@ -520,7 +521,6 @@ static int gemm_rs_impl(MtComm* c, void* stream, const void* const* A, const voi
     a.tb = tb;
     a.ncomm = (nred + 1) & ~1;
     const int nclusters = (grid - a.ncomm) / 2;
-    if (nclusters < 1) return fail("nred out of range");
     cudaError_t e2 = mt::launch_gemm_pair(mt::MODE_GEMM_RS, maps, sf, a, nclusters, c->nlocal, (cudaStream_t)stream, fp8);
     if (e2 != cudaSuccess) return fail(std::string("pair gemm_rs launch: ") + cudaGetErrorString(e2));
     mthost::stat_add(mthost::ST_GEMM_RS, (uint64_t)(2.0 * M * N * K));

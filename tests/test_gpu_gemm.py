@@ -318,3 +318,28 @@ def test_128_leftover_rows_give_the_bits_of_pairs(shape, monkeypatch):
         monkeypatch.delenv("MINTCCL_GEMM_BN")
         assert torch.equal(chosen, pairs) and torch.equal(few, pairs)
     close(G.gemm(a, w), ref_mm(a, w), K)
+
+
+def test_one_rank_plans_refuse_what_the_fused_kernels_do():
+    """One CTA is no pair, and the reducers of the C interface have to leave one: refused although nothing is gathered or
+    reduced at one rank.  128 rows run on single CTAs, where one is enough."""
+    from mintccl_b200 import _native as N
+    from mintccl_b200.ops.gemm import AllGatherGemm, GemmReduceScatter
+    w_ = world(1)
+    for rows, refused in ((256, True), (128, False)):
+        a = torch.zeros(rows, 128, device="cuda", dtype=torch.bfloat16)
+        b = torch.zeros(256, 128, device="cuda", dtype=torch.bfloat16)
+        for plan in (AllGatherGemm(w_, rows, 256, 128), GemmReduceScatter(w_, rows, 256, 128)):
+            if refused:
+                with pytest.raises(RuntimeError, match="CTAs|nred"):
+                    plan([a], [b], nctas=1)
+            else:
+                assert bool((plan([a], [b], nctas=1)[0] == 0).all())
+    out = torch.empty(256, 256, device="cuda", dtype=torch.bfloat16)
+    a = torch.zeros(256, 128, device="cuda", dtype=torch.bfloat16)
+    ptrs = [N.ptr_array([t.data_ptr()]) for t in (a, b, out)]
+    lib, args = w_.lib, (0, 0, 1, 256, 256, 128)
+    for nred, nctas in ((-1, 0), (148, 0), (3, 4)):
+        assert lib.mt_gemm_rs(w_._handle, w_._stream(), *ptrs, *args, nred, nctas) == -1
+        assert "nred" in N.last_error()
+    assert lib.mt_ag_gemm(w_._handle, w_._stream(), *ptrs, *args, 256, 0, 0, 4, 0, 1) == -1
