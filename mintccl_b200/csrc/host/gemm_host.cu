@@ -380,7 +380,7 @@ static int ag_gemm_impl(MtComm* c, void* stream, const void* const* a_shard, con
     if (n > 1 && (!use_pair(M / n) || comm_mode == 2)) return fail("the fused activation runs on CTA pairs");
   }
   if (comm_mode < 0 || comm_mode > 3) return fail("comm_mode must be 0, 1, 2 or 3");
-  if (n == 1 && (pair_on() || act)) {   // nothing to gather: the product itself
+  if (n == 1) {   // nothing to gather: the product itself (gather_off, flags_off and epoch are not looked at)
     if (nctas == 1 && use_pair(M) && comm_mode != 2) return fail("not enough CTAs for the requested comm CTAs");
     if (((uintptr_t)C[0] & 15) || (fp8 && (((uintptr_t)sfa[0] | (uintptr_t)sfb[0]) & 15))) return fail("C and the scales must be 16-byte aligned");
     if (!act)
@@ -389,8 +389,7 @@ static int ag_gemm_impl(MtComm* c, void* stream, const void* const* a_shard, con
     return gemm_pair(stream, a_shard[0], nullptr, B[0], nullptr, C[0], M, N, K, ldc, nctas, false, mthost::ST_AG_GEMM, waits_of(a),
                      false, false, a.epi, a.aux[0]);
   }
-  if (n == 1) ncomm = 0;
-  else if (ncomm < 1 || ncomm > 64) return fail("ncomm out of range");
+  if (ncomm < 1 || ncomm > 64) return fail("ncomm out of range");
   int grid = nctas > 0 ? nctas : sm_count(c->device);
   if (c->emulated && grid * c->nlocal > sm_count(c->device)) grid = sm_count(c->device) / c->nlocal;
   if (grid <= ncomm) return fail("not enough CTAs for the requested comm CTAs");
@@ -399,8 +398,8 @@ static int ag_gemm_impl(MtComm* c, void* stream, const void* const* a_shard, con
   a.ncomm = ncomm;
   a.gather_off = gather_off;
   a.comm_mode = comm_mode;
-  if (n > 1 && (comm_split < 1 || comm_split > ncomm)) return fail("comm_split must be in [1, ncomm]");
-  a.comm_split = n > 1 ? comm_split : 1;
+  if (comm_split < 1 || comm_split > ncomm) return fail("comm_split must be in [1, ncomm]");
+  a.comm_split = comm_split;
   a.shard_off = shard_off;
   mt::GemmMaps maps;
   memset(&maps, 0, sizeof(maps));
@@ -484,7 +483,8 @@ static int gemm_rs_impl(MtComm* c, void* stream, const void* const* A, const voi
   if (nred < 0 || nred >= grid || (use_pair(M / c->nranks) && grid - ((nred + 1) & ~1) < 2)) return fail("nred out of range");
   if (c->nranks == 1) {
     // nothing to reduce: the product itself, without the staging area and the reducers' pass over it (8192 x 4096 x 1792:
-    // 128 us with them, 83 without).  The sum of one bf16 partial tile is that tile, so the bytes are the same.
+    // 128 us with them, 83 without; stage_off, flags_off and epoch are not looked at).  The sum of one bf16 partial tile is
+    // that tile.
     if ((uintptr_t)out[0] & 15) return fail("out must be 16-byte aligned");
     if (fp8 && (((uintptr_t)sfa[0] | (uintptr_t)sfb[0]) & 15)) return fail("scale tensors must be 16-byte aligned");
     if (tb)

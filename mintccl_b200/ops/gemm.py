@@ -124,7 +124,8 @@ class AllGatherGemm(_Fused):
         self.M, self.N, self.K, self.ncomm = M, N_, K, ncomm
         if fp8 and K % 128:
             raise ValueError("MXFP8: K must be a multiple of 128")
-        self.gathered = comm.symm_empty((M, K), torch.uint8 if fp8 else torch.bfloat16)
+        # one rank gathers nothing: a placeholder, so that the plan's buffers are freed alike
+        self.gathered = comm.symm_empty((M, K) if n > 1 else (1, 1), torch.uint8 if fp8 else torch.bfloat16)
         # MXFP8: the tiled scales of all ranks' rows, gathered by a small all-gather before the fused kernel
         self.sfa_all = comm.symm_empty((n, (M // n // 128) * (K // 128) * 512), torch.uint8) if fp8 else None
         self.flags = comm.symm_zeros((n * (M // n // BM),), torch.int64)
@@ -234,8 +235,8 @@ class GemmReduceScatter(_Fused):
             nred = self.pick_nred(M, N_, K, n)
         self.nred = nred if n > 1 else 0
         # two halves used alternately: a fast peer may already write the next call's partial tiles while this
-        # rank still reduces the current ones
-        self.stage = comm.symm_empty((2, n, M // n, N_), torch.bfloat16)
+        # rank still reduces the current ones.  One rank stages nothing: a placeholder, so that the plan's buffers are freed alike
+        self.stage = comm.symm_empty((2, n, M // n, N_) if n > 1 else (1, 1), torch.bfloat16)
         self.flags = comm.symm_zeros((n * (M // n // BM) * (N_ // BN) + 2,), torch.int64)
         torch.cuda.synchronize()
         comm.control.barrier()

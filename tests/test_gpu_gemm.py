@@ -343,3 +343,22 @@ def test_one_rank_plans_refuse_what_the_fused_kernels_do():
         assert lib.mt_gemm_rs(w_._handle, w_._stream(), *ptrs, *args, nred, nctas) == -1
         assert "nred" in N.last_error()
     assert lib.mt_ag_gemm(w_._handle, w_._stream(), *ptrs, *args, 256, 0, 0, 4, 0, 1) == -1
+
+
+@pytest.mark.parametrize("rows", [128, 512])
+def test_one_rank_plans_leave_the_heap_alone(rows, gemm_kernel):
+    """What they do not gather or stage is not allocated either, and they still give the product."""
+    from mintccl_b200.ops.gemm import AllGatherGemm, GemmReduceScatter
+    w_ = world(1)
+    used = sum(w_._allocs.values())
+    ag, rs = AllGatherGemm(w_, rows, 512, 1024), GemmReduceScatter(w_, rows, 512, 1024)
+    assert sum(w_._allocs.values()) - used <= 4 * 256
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    a = torch.randn(rows, 1024, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(512, 1024, generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    for plan in (ag, rs):
+        close(plan([a], [w])[0], ref_mm(a, w), 1024)
+    w_.check()
+    for t in (ag.gathered, ag.flags, rs.stage, rs.flags):
+        w_.symm_free(t)
+    assert sum(w_._allocs.values()) == used
