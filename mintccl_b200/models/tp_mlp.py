@@ -18,6 +18,12 @@ import torch
 from ..ops.gemm import AllGatherGemm, GemmReduceScatter, gemm_dsilu, gemm_t
 
 
+def _operand(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as TMA takes it: contiguous, on a 16-byte boundary.  A saved tensor is what a saved-tensor hook made of it."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _MLPFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x_shard, w_up, w_down, mlp):
@@ -31,7 +37,7 @@ class _MLPFunction(torch.autograd.Function):
     def backward(ctx, dy_shard):
         mlp = ctx.mlp
         comm = mlp.comm
-        x_shard, w_up, w_down, h, a = ctx.saved_tensors
+        x_shard, w_up, w_down, h, a = map(_operand, ctx.saved_tensors)
         n, T = comm.world_size, mlp.tokens
         dy_shard = dy_shard.contiguous()
         # all-gather dy and x over tokens (plain collectives of this library)

@@ -362,3 +362,40 @@ def test_one_rank_plans_leave_the_heap_alone(rows, gemm_kernel):
     for t in (ag.gathered, ag.flags, rs.stage, rs.flags):
         w_.symm_free(t)
     assert sum(w_._allocs.values()) == used
+
+
+def one_rank_mlp(T, H, F):
+    import mintccl_b200
+    from mintccl_b200 import Config
+    from mintccl_b200.models.tp_mlp import TensorParallelMLP
+    from mintccl_b200.parallel.rendezvous import SingleControl
+    cfg = Config.from_env(max_channels=2, num_blocks=2, buff_size=1 << 20, heap_bytes=64 << 20, scratch_bytes=1 << 20,
+                          wait_timeout_ms=4000)
+    comm = mintccl_b200.Communicator(control=SingleControl(), device=0, config=cfg)
+    return comm, TensorParallelMLP(comm, T, H, F)
+
+
+def mlp_step(mlp, x, dy):
+    x = x.detach().requires_grad_(True)
+    y = mlp(x)
+    return (y.detach(), *torch.autograd.grad(y, [x, mlp.w_up, mlp.w_down], dy))
+
+
+@pytest.mark.parametrize("form", ["strided", "misaligned"])
+def test_mlp_backward_takes_saved_tensors_in_any_layout(form):
+    """A saved-tensor hook may hand a tensor back in another layout or off the 16-byte grid."""
+    T, H, F = 384, 256, 512
+    comm, mlp = one_rank_mlp(T, H, F)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x, dy = (torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    want = mlp_step(mlp, x, dy)
+
+    def unpack(t):
+        if form == "strided":
+            return t.t().contiguous().t()
+        return torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view(t.shape)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        got = mlp_step(mlp, x, dy)
+    comm.check()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    comm.close()
