@@ -29,7 +29,7 @@ class _MLPFunction(torch.autograd.Function):
     def forward(ctx, x_shard, w_up, w_down, mlp):
         h, a = mlp.ag_gemm.call_silu(x_shard, w_up)          # [T, F/n], and silu of it
         y = mlp.gemm_rs(a, w_down)                           # [T/n, H]
-        ctx.mlp = mlp
+        ctx.mlp, ctx.epoch = mlp, mlp.ag_gemm.epoch
         ctx.save_for_backward(x_shard, w_up, w_down, h, a)
         return y
 
@@ -40,12 +40,18 @@ class _MLPFunction(torch.autograd.Function):
         x_shard, w_up, w_down, h, a = map(_operand, ctx.saved_tensors)
         n, T = comm.world_size, mlp.tokens
         dy_shard = dy_shard.contiguous()
-        # all-gather dy and x over tokens (plain collectives of this library)
+        # all-gather dy and x over tokens (plain collectives of this library); x is still in the plan's buffer, but for this
+        # rank's own rows, unless another forward pass went through the plan since (the same answer on every rank)
         dy = mlp._gather(dy_shard)                           # [T, H]
-        x = mlp.ag_gemm.gathered if n > 1 else x_shard       # gathered x is still in the plan's buffer
-        if n > 1:
-            x = x.clone()
+        if n == 1:
+            x = x_shard
+        elif mlp.ag_gemm.epoch == ctx.epoch:
+            x = mlp.ag_gemm.gathered.clone()
             x[comm.rank * (T // n):(comm.rank + 1) * (T // n)].copy_(x_shard)
+        else:
+            x = x_shard.new_empty((n, *x_shard.shape))
+            comm.allgather(x, inp=x_shard)
+            x = x.view(T, -1)
         dh = gemm_dsilu(dy, w_down, h)                       # [T, F/n] = (dy @ w_down) * silu'(h)   (w_down: [H, F/n])
         dw_down = gemm_t(dy, a, ta=True, tb=True)            # [H, F/n] = dy^T @ a
         dw_up = gemm_t(dh, x, ta=True, tb=True)              # [F/n, H] = dh^T @ x
