@@ -1,9 +1,9 @@
 """Tensor-parallel MLP on the fused kernels: all-gather -> GEMM and GEMM -> reduce-scatter in one launch each.
 
 Run:  python -m mintccl_b200.launch -np 2 examples/10_fused_tp_mlp.py     (or torchrun; one process per GPU)
-Needs GPUs (tcgen05 kernels); on a machine without CUDA it says so and exits 0.  The forward pass is checked
-against the same block computed without tensor parallelism in fp32, the MXFP8 projection against the product
-of the dequantised operands.  MINTCCL_TEST_COUNT sets the number of tokens (rounded to 256 x world).
+Needs GPUs (tcgen05 kernels); on a machine without CUDA it says so and exits 0.  The forward pass and the gradients
+are checked against the same block computed without tensor parallelism in fp32, the MXFP8 projection against the
+product of the dequantised operands.  MINTCCL_TEST_COUNT sets the number of tokens (rounded to 256 x world).
 """
 import os
 import sys
@@ -47,15 +47,21 @@ mlp = TensorParallelMLP(comm, T, H, F)
 x_full = torch.randn(T, H, generator=torch.Generator().manual_seed(7)).to(torch.bfloat16).cuda()
 x_shard = x_full[rank * (T // world):(rank + 1) * (T // world)].clone().requires_grad_(True)
 y_shard = mlp(x_shard)                                        # [T / world, H]
-y_shard.float().pow(2).mean().backward()
+dy_full = torch.randn(T, H, generator=torch.Generator().manual_seed(8)).to(torch.bfloat16).cuda()
+rows = slice(rank * (T // world), (rank + 1) * (T // world))
+y_shard.backward(dy_full[rows])
 torch.cuda.synchronize()
 comm.check()
 w_up = gather(mlp.w_up.detach())                              # [F, H]: the column-parallel weight, whole
 w_down = gather(mlp.w_down.detach().t().contiguous()).t()     # [H, F]: the row-parallel weight, whole
-ref = torch.nn.functional.silu(x_full.float() @ w_up.float().t()) @ w_down.float().t()
-mine = ref[rank * (T // world):(rank + 1) * (T // world)]
-check("fused MLP forward", torch.allclose(y_shard.detach().float(), mine, rtol=5e-2, atol=5e-2))
-check("gradients", all(g is not None and bool(torch.isfinite(g.float()).all()) for g in (x_shard.grad, mlp.w_up.grad, mlp.w_down.grad)))
+xr, up, down = (t.float().requires_grad_(True) for t in (x_full, w_up, w_down))
+ref = torch.nn.functional.silu(xr @ up.t()) @ down.t()
+check("fused MLP forward", torch.allclose(y_shard.detach().float(), ref.detach()[rows], rtol=5e-2, atol=5e-2))
+dx, dup, ddown = torch.autograd.grad(ref, [xr, up, down], dy_full.float())
+cols = slice(rank * (F // world), (rank + 1) * (F // world))  # this rank's part of either weight
+for what, got, want in (("input", x_shard.grad, dx[rows]), ("up projection", mlp.w_up.grad, dup[cols]),
+                        ("down projection", mlp.w_down.grad, ddown[:, cols])):
+    check(f"gradient of the {what}", float((got.float() - want).norm() / want.norm()) < 1e-2)
 
 # ---- the up projection on block-scaled fp8 operands (e4m3 payload, one power-of-two scale per 32 elements)
 plan = AllGatherGemm(comm, T, F // world, H, fp8=True)

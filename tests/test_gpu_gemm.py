@@ -16,8 +16,9 @@ def close(got, ref32, k):
 
 @pytest.fixture(params=[1, 0], ids=["cta_pair", "single_cta"])
 def gemm_kernel(request):
-    """Plain GEMMs run on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles) when M % 256 == 0, else on the
-    single-CTA kernel (128 x 256 tiles); both are tested on every shape."""
+    """Plain GEMMs run on CTA pairs (tcgen05 cta_group::2, 256 rows and 64 to 256 columns a tile), or on the
+    single-CTA kernel (128 x 256 tiles) with MINTCCL_GEMM_PAIR=0 and where 128 leftover rows make that faster; every shape
+    is tested with both settings."""
     from mintccl_b200 import _native as N
     N.lib().mt_gemm_set_pair(request.param)
     yield request.param
@@ -398,4 +399,24 @@ def test_mlp_backward_takes_saved_tensors_in_any_layout(form):
         got = mlp_step(mlp, x, dy)
     comm.check()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+    comm.close()
+
+
+@pytest.mark.parametrize("T,H,F", [(384, 256, 512), (1024, 512, 1792)])
+def test_mlp_gradients_against_autograd(T, H, F, gemm_kernel):
+    """Forward and gradients of the block against fp32 autograd on the same bf16 inputs; 384 tokens leave 128 rows over.
+    Up to four values on a path are rounded to bf16 (h, its activation, the two gradients behind them, the result), each
+    2^-9 at most of its size: 2-norms within 8e-3 of the result's."""
+    comm, mlp = one_rank_mlp(T, H, F)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x, dy = (torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    with torch.no_grad():
+        mlp.w_up.copy_(torch.randn(F, H, generator=g, device="cuda") * H ** -0.5)
+        mlp.w_down.copy_(torch.randn(H, F, generator=g, device="cuda") * F ** -0.5)
+    got = mlp_step(mlp, x, dy)
+    comm.check()
+    xr, up, down = (t.detach().float().requires_grad_(True) for t in (x, mlp.w_up, mlp.w_down))
+    y = torch.nn.functional.silu(xr @ up.t()) @ down.t()
+    for a, b in zip(got, (y.detach(), *torch.autograd.grad(y, [xr, up, down], dy.float()))):
+        assert float((a.float() - b).norm() / b.norm()) < 8e-3
     comm.close()
