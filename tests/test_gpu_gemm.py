@@ -253,6 +253,9 @@ def test_silu_of_every_finite_bf16():
     assert torch.equal(hs[0], v)
     assert torch.equal(acts[0], torch.nn.functional.silu(v))
     assert bool((acts[0][(v < -87.4) & (v > -88.6)] != 0).all())
+    hs, acts = AllGatherGemm(w_, T, F, T).call_silu([torch.eye(T, device="cuda").to(torch.bfloat16) * 3e38], [v.t().contiguous()])
+    assert bool(hs[0].isposinf().any()) and bool(hs[0].isneginf().any())
+    assert same(acts[0], torch.nn.functional.silu(hs[0]))
 
 
 @pytest.mark.parametrize("shape", [(128, 256, 64), (128, 512, 64), (384, 1792, 128), (8192, 1792, 256), (2048, 512, 448)])
