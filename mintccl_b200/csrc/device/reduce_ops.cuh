@@ -147,10 +147,6 @@ template <>
 __device__ __forceinline__ uint8_t float_to_elem<U8>(float v) { return (uint8_t)v; }
 
 // ---- MXFP8 (e4m3 payload, ue8m0 scale per 32 elements) ----------------------------------------------
-__device__ __forceinline__ float e4m3_to_float(uint8_t v) {
-  __half_raw h = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)v, __NV_E4M3);
-  return __half2float(*reinterpret_cast<__half*>(&h));
-}
 __device__ __forceinline__ uint8_t float_to_e4m3(float f) {
   return (uint8_t)__nv_cvt_float_to_fp8(f, __NV_SATFINITE, __NV_E4M3);
 }

@@ -143,9 +143,13 @@ static int pick_bn(int row_tiles, int N, int nclusters, bool fp8) {
 }
 // The same for a plain GEMM, where narrow tiles are to be had too.  The time of a wave in tenths of a 256-column k-block
 // (580 cycles): 9 a k-block for 224 columns, 5.5 for 128 (290 - 320 cycles), 4 for 64 (220: A's bytes do not shrink with
-// the tile), and one k-block to drain the last accumulator.  So a problem with too few wide tiles for the chip takes
-// the widest ones that fill it.  Measured (us, 256 / 128 / 64 columns): 128 x 4096 x 1792 13.7 / 9.1 / 7.9,
-// 512 x 4096 x 1792 14.5 / 9.9 / 12.1, 1024 x 1792 x 4096 24.8 / 15.6 / 20.5, 2048 x 4096 x 2048 26.3 / 25.3 / 33.0.
+// the tile), and one k-block to drain the last accumulator; an MXFP8 k-block of 128 elements has the same ratios.  So a
+// problem with too few wide tiles for the chip takes the widest ones that fill it.  Of 204 shapes of whole 256-row blocks
+// (256, 2048 and 8192 rows, 256 - 14336 columns, K = 256 - 8192, both types), timed in every width, the choice is within 5 %
+// of the best for all but one (8192 x 14336 x 256: 9 %).  Measured (us, 256 / 128 / 64 columns): 256 x 4096 x 2048 16.6 /
+// 12.5 / 10.4, 2048 x 1024 x 4096 27.1 / 18.6 / 23.3, 2048 x 4096 x 2048 28.9 / 28.8 / 37.1, 8192 x 1792 x 4096 90.1 / 87.6 /
+// 117.4 (224: 84.6); MXFP8 (256 / 128) 256 x 1792 x 4096 16.6 / 11.3, 8192 x 1792 x 4096 51.3 / 48.5, 8192 x 4096 x 2048
+// 53.8 / 57.1.
 static int pick_plain_bn(int row_tiles, int N, int kblocks, int nclusters, bool fp8, bool tb, long* cost_out = nullptr) {
   if (const int f = forced_bn(N, fp8, true, tb)) return f;
   const int wide = pick_wide(row_tiles, N, nclusters, fp8);

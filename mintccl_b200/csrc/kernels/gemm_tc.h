@@ -57,8 +57,9 @@ struct GemmArgs {
 cudaError_t launch_gemm_tc(int mode, const GemmMaps& maps, const GemmArgs& a, int nctas, int nlocal, cudaStream_t s,
                            bool fp8 = false);
 
-// ---- GEMM on CTA pairs (gemm_tc2.cu): one 256 x 256 tile per cluster of two CTAs, same modes and arguments ----
-// GemmMaps for this kernel: boxes of 128 rows x 128 bytes for A and for B (each CTA of a pair loads half of B).
+// ---- GEMM on CTA pairs (gemm_tc2.cu): one tile of 256 rows per cluster of two CTAs, same modes and arguments ----
+// GemmMaps for this kernel: boxes of 128 rows x 128 bytes for A, bn / 2 rows x 128 bytes for B (each CTA of a pair loads
+// half of B); 64 columns x 64 K rows for an operand stored transposed.
 template <int NR>
 struct PairSfMapsN {
   CUtensorMap sfa[NR];  // MXFP8: tiled scales of (the gathered) A as [atoms, 128] u32, box = one 512-byte atom
@@ -66,7 +67,7 @@ struct PairSfMapsN {
 };
 typedef PairSfMapsN<MT_MAX_RANKS> PairSfMaps;
 // bn: columns of a tile: 256, 224 (bf16, plain GEMM and all-gather -> GEMM), 128 (plain GEMM), 64 (bf16 plain GEMM, B
-// K-major); the map of B has boxes of bn / 2 rows
+// K-major)
 cudaError_t launch_gemm_pair(int mode, const GemmMaps& maps, const PairSfMaps& sf, const GemmArgs& a, int nclusters,
                              int nlocal, cudaStream_t s, bool fp8, int bn = 256);
 int gemm_pair_max_clusters(int mode, bool fp8, int bn = 256, int form = 0);

@@ -1,23 +1,28 @@
 // GEMM on CTA pairs: C[M, N] = A[M, K] * B[N, K]^T with tcgen05.mma.cta_group::2.
 //
-// Two CTAs of one cluster (neighbouring SMs) compute one 256 x 256 tile.  Each CTA stages 128 rows of A and
-// 128 rows of B per K block, so the tensor cores of both SMs read every B row from ONE shared memory only:
-// per SM and MMA, the shared-memory traffic (TMA writes + operand reads) drops from 24 KiB to 16 KiB compared
-// with the single-CTA 128 x 256 tile of gemm_tc.cu, and a stage takes 32 KiB instead of 48, which pays for a
-// 6-deep ring.  The leader CTA (cluster rank 0) issues every MMA; the accumulator rows [0, 128) live in the
-// leader's TMEM and [128, 256) in the peer's, and each CTA's epilogue warps drain their own half.
+// Two CTAs of one cluster (neighbouring SMs) compute one tile of 256 rows and 256, 224, 128 or 64 columns (the widths:
+// see gemm_pair_kernel).  Each CTA stages 128 rows of A and half the tile's rows of B per K block, so the tensor cores of
+// both SMs read every B row from ONE shared memory only: at 256 columns, per SM and MMA, the shared-memory traffic (TMA
+// writes + operand reads) drops from 24 KiB to 16 KiB compared with the single-CTA 128 x 256 tile of gemm_tc.cu, and a
+// stage takes 32 KiB instead of 48, which pays for a 6-deep ring (8 and 10 deep for 128 and 64 columns).  The leader CTA
+// (cluster rank 0) issues every MMA; the accumulator rows [0, 128) live in the leader's TMEM and [128, 256) in the peer's,
+// and each CTA's epilogue warps drain their own half.
 //
 //   warp 0 (both CTAs)  TMA producer: own halves of A and B (and the MXFP8 scale atoms) into own shared
 //                       memory; the bytes of both CTAs are counted on the LEADER's "stage full" barrier
-//   warp 1 (leader)     one lane issues tcgen05.mma for the pair and commits to the leader's "stage empty" and
-//                       "accumulator full" barriers; the leader's producer / first epilogue warp pass each
-//                       of these on to the peer's barrier with a remote mbarrier arrive
-//   warps 2..5 (both)   epilogue: TMEM -> registers -> bf16 -> shared memory -> global memory; every warp
-//                       arrives on the leader's "accumulator empty" barrier (8 arrivals per tile)
+//   warp 1 (leader)     issues tcgen05.mma for the pair and commits to the leader's "stage empty" and "accumulator
+//                       full" barriers; the leader's producer / first epilogue warp pass each of these on to the
+//                       peer's barrier with a remote mbarrier arrive
+//   warps 2..5 (both)   epilogue: TMEM -> registers -> bf16 -> shared memory -> whole lines in global memory; with an
+//                       activation straight from the registers, in 32-byte sectors; every warp arrives on the
+//                       leader's "accumulator empty" barrier (8 arrivals per tile)
+//
+// Warps 0 and 1 run their loops uniformly, with all lanes waiting; one elected lane issues.
 //
 // Every wait is bounded; on expiry the CTA raises its abort flag, all roles leave their loops, both CTAs meet
 // at the closing cluster barrier (so neither exits while the other may still signal into it), TMEM is
-// released and a device-side error word is set for the host.  No load is replicated across the cluster.
+// released and a device-side error word is set for the host, the communicator's status record too where the launch
+// has one (the fused modes and the product of a one-rank plan).  No load is replicated across the cluster.
 //
 // Modes (as in gemm_tc.cu): the plain GEMM; all-gather -> GEMM, where extra CTAs of the grid move the peers' rows
 // into local memory and each producer waits for the arrival counter of its own 128 rows; GEMM -> reduce-scatter,
