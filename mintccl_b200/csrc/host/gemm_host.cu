@@ -261,13 +261,15 @@ static int gemm_single(void* stream, const void* A, const void* sfa, const void*
 // C[M, ldc] = A[M, K] * B[N, K]^T, both K-major, on the kernel that suits the shape.  A last block of 128 rows leaves half a
 // pair idle, and 128-row tiles of single CTAs can need a wave less (1152 x 4096: 144 tiles on 148 SMs; pairs have 80 on 74
 // clusters).  In pick_plain_bn's unit (twice the tenths of a 256-column k-block) a wave of single CTAs costs 23 a k-block
-// and 5 (10 in MXFP8) for the drain; a lone bf16 wave 20.4 and 20 less, since nothing waits for its accumulator.  Of 418
-// shapes with 128 leftover rows (128 - 4224 x 256 - 14336, K = 256 - 8192, both types), timed on both kernels, four lose
-// 5 % by this choice and the others at most 3.  1152 x 4096 x 4096 takes 28.9 us (pairs 38.0), MXFP8 1152 x 4096 x 1024 10.4
-// (12.5), 640 x 4096 x 4096 26.8 (28.8); 2176 x 14336 x 1024 stays on pairs: 49.0, single CTAs 54.1.
+// and 5 (10 in MXFP8) for the drain; a lone bf16 wave 20.7 and 24 less, since nothing waits for its accumulator.  Of 418
+// shapes with 128 leftover rows (128 - 4224 x 256 - 14336, K = 256 - 8192, both types), timed on both kernels with operands
+// in the L2, six lose 4 - 7 % by this choice and the others at most 3.  1152 x 4096 x 4096 takes 28.9 us (pairs 38.0), MXFP8
+// 1152 x 4096 x 1024 10.4 (12.5); 2176 x 14336 x 1024 stays on pairs: 49.0, single CTAs 54.1.  A lone wave is left to pairs
+// from K = 4096 on, where operands that come from HBM decide: 640 x 4096 x 4096 28.8 us on pairs and 30.8 on single CTAs
+// (28.8 and 26.8 out of the L2), 4224 x 1024 x 4096 29.7 and 31.9.
 static long single_cost(int M, int N, int kblocks, int sms, bool fp8) {
   const long waves = ((long)(M / kBM) * (N / kBN) + sms - 1) / sms;
-  if (waves == 1 && !fp8) return kblocks * 102L / 5 - 20;
+  if (waves == 1 && !fp8) return kblocks * 207L / 10 - 24;
   return waves * (kblocks * 23L + (fp8 ? 10 : 5));
 }
 static int gemm_plain(void* stream, const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N, int K,
