@@ -2,6 +2,7 @@
 tensor core reads.  The GPU kernels are checked against these functions in the gpu-marked tests."""
 import pytest
 import torch
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from mintccl_b200.ops import mxfp8 as mx
 
@@ -89,7 +90,7 @@ class _Sub(torch.Tensor):
     pass
 
 
-class _Mode(torch.utils._python_dispatch.TorchDispatchMode):
+class _Mode(TorchDispatchMode):
     def __torch_dispatch__(self, func, types, args=(), kwargs=None):
         return func(*args, **(kwargs or {}))
 
@@ -112,7 +113,7 @@ def test_traced_encoding_replays_on_other_inputs(no_kernels):
     g = torch.Generator().manual_seed(5)
     x, y = torch.randn(128, 128, generator=g), torch.randn(128, 128, generator=g) * 40.0
     sx, sy = (torch.randint(0, 256, (128, 8), generator=g, dtype=torch.uint8) for _ in range(2))
-    make_fx = torch.fx.experimental.proxy_tensor.make_fx
+    from torch.fx.experimental.proxy_tensor import make_fx
     for got, want in zip(make_fx(mx.quantize_rows_mxfp8)(x)(y), mx._torch_quantize(y)):
         assert torch.equal(got.reshape(-1), want)
     for f in (make_fx(mx.tile_scales)(sx), torch.jit.trace(mx.tile_scales, sx, check_trace=False)):
